@@ -14,6 +14,8 @@
 // A thread owns one plane cell and kFoldF frequencies: their sums stay in registers for the
 // whole window, the staged values of consecutive cells are coalesced, and the (cos, sin) table
 // row of each step is a broadcast.
+#include <type_traits>
+
 #include "fdtd_kernels.cuh"
 
 namespace fdtd {
@@ -37,18 +39,37 @@ __device__ __forceinline__ void fold_monitor(const MonitorDev& m, const Grid& g,
     im[q] = q < nfc ? m.im[(long long)(f0 + q) * np + p] : 0.0;
   }
   const float* st = m.stage + p;
-  for (int s = 0; s < n; ++s) {
-    const long long t = t0 + s;
-    const double v = (double)st[(t & (kDftSlots - 1)) * np];
-    const double2* tab = m.tab + t * m.nf + f0;
+  const double scale = m.scale;
+  const int nf = m.nf;
+  const double2* tab0 = m.tab + t0 * nf + f0;
+  const int slot0 = (int)(t0 & (kDftSlots - 1));
+  // x * 1.0 == x: without a scale two of the six operations per step and frequency fall away.
+  auto window = [&](auto scaled, auto full) {
+#pragma unroll 4
+    for (int s = 0; s < n; ++s) {
+      const double v = (double)st[(long long)((slot0 + s) & (kDftSlots - 1)) * np];
+      const double2* tab = tab0 + (long long)s * nf;
 #pragma unroll
-    for (int q = 0; q < kFoldF; ++q) {
-      if (q < nfc) {
-        const double2 cs = __ldg(&tab[q]);
-        re[q] = dadd(re[q], dmul(dmul(v, cs.x), m.scale));
-        im[q] = dsub(im[q], dmul(dmul(v, cs.y), m.scale));
+      for (int q = 0; q < kFoldF; ++q) {
+        if (decltype(full)::value || q < nfc) {
+          const double2 cs = __ldg(&tab[q]);
+          double c = dmul(v, cs.x), d = dmul(v, cs.y);
+          if (decltype(scaled)::value) {
+            c = dmul(c, scale);
+            d = dmul(d, scale);
+          }
+          re[q] = dadd(re[q], c);
+          im[q] = dsub(im[q], d);
+        }
       }
     }
+  };
+  using Yes = std::true_type;
+  using No = std::false_type;
+  if (scale == 1.0) {
+    if (nfc == kFoldF) window(No{}, Yes{}); else window(No{}, No{});
+  } else {
+    if (nfc == kFoldF) window(Yes{}, Yes{}); else window(Yes{}, No{});
   }
 #pragma unroll
   for (int q = 0; q < kFoldF; ++q) {
@@ -65,19 +86,33 @@ __global__ void __launch_bounds__(kFoldThreads) dft_fold(const __grid_constant__
   if ((int)blockIdx.z < M.n) fold_monitor(M.m[blockIdx.z], g, t0, n);
 }
 
-// A batch: blockIdx.z is the grid; its arguments (monitors, step counter t0 at the start of the
+// A batch: blockIdx.z is grid * kMaxMonitors + monitor; the grid's arguments (monitors, step counter t0 at the start of the
 // batch step) are the ones the batched kernel reads (TiledArgs, or CpmlSim for CPML batches).
 // The window starts t_offset steps later.
 template <class Args>
 __global__ void __launch_bounds__(kFoldThreads) dft_fold_batch(const Args* grids,
                                                                long long t_offset, int n) {
-  const Args& a = grids[blockIdx.z];
-  for (int k = 0; k < a.M.n; ++k) fold_monitor(a.M.m[k], a.g, a.t0 + t_offset, n);
+  const Args& a = grids[blockIdx.z / kMaxMonitors];
+  const int k = (int)blockIdx.z % kMaxMonitors;
+  if (k < a.M.n) fold_monitor(a.M.m[k], a.g, a.t0 + t_offset, n);
 }
 
 dim3 fold_grid(long long max_np, int max_nf, int nz) {
   return dim3((unsigned)((max_np + kFoldThreads - 1) / kFoldThreads),
               (unsigned)((max_nf + kFoldF - 1) / kFoldF), (unsigned)nz);
+}
+
+// Launches of as many grids as blockIdx.z can number.
+template <class Args>
+cudaError_t fold_batch(const Args* grids, int ngrids, long long max_np, int max_nf,
+                       long long t_offset, int n, cudaStream_t st) {
+  constexpr int per = 65535 / kMaxMonitors;
+  for (int g0 = 0; g0 < ngrids; g0 += per) {
+    const int ng = ngrids - g0 < per ? ngrids - g0 : per;
+    dft_fold_batch<Args><<<fold_grid(max_np, max_nf, ng * kMaxMonitors), kFoldThreads, 0, st>>>(
+        grids + g0, t_offset, n);
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -95,19 +130,15 @@ cudaError_t launch_dft_fold(const Monitors& M, const Grid& g, long long t0, int 
 cudaError_t launch_dft_fold_batch(const TiledArgs* grids, int ngrids, long long max_np,
                                   int max_nf, long long t_offset, int n, cudaStream_t st) {
   if (ngrids <= 0 || max_nf <= 0 || n <= 0) return cudaSuccess;
-  if (n > kDftSlots || t_offset < 0 || ngrids > 65535) return cudaErrorInvalidValue;
-  dft_fold_batch<TiledArgs>
-      <<<fold_grid(max_np, max_nf, ngrids), kFoldThreads, 0, st>>>(grids, t_offset, n);
-  return cudaGetLastError();
+  if (n > kDftSlots || t_offset < 0) return cudaErrorInvalidValue;
+  return fold_batch(grids, ngrids, max_np, max_nf, t_offset, n, st);
 }
 
 cudaError_t launch_dft_fold_cpml_batch(const CpmlSim* sims, int nsims, long long max_np,
                                        int max_nf, long long t_offset, int n, cudaStream_t st) {
   if (nsims <= 0 || max_nf <= 0 || n <= 0) return cudaSuccess;
-  if (n > kDftSlots || t_offset < 0 || nsims > 65535) return cudaErrorInvalidValue;
-  dft_fold_batch<CpmlSim>
-      <<<fold_grid(max_np, max_nf, nsims), kFoldThreads, 0, st>>>(sims, t_offset, n);
-  return cudaGetLastError();
+  if (n > kDftSlots || t_offset < 0) return cudaErrorInvalidValue;
+  return fold_batch(sims, nsims, max_np, max_nf, t_offset, n, st);
 }
 
 }  // namespace fdtd
