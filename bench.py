@@ -347,7 +347,7 @@ def run_ours(args):
     sim.set_coefficients(coefs)
     sim.set_fast_path(not args.no_fast_path)
     if args.cpml:
-        # the tiled kernel plus the shell companion (per-step kernels when the grid is small)
+        # per-step kernels, or with --blt the tiled kernel plus the shell companion
         sim.set_cpml(thickness=args.cpml)
     sim.set_sources(src)
     mid = sim.add_dft_monitor("Ez", nz // 2, freqs, scale=1.0)
@@ -716,8 +716,8 @@ def cpml_results(L=10, reps=2):
     wave = W.gaussian_wave(T)
     freqs = W.source_band(N_FREQS)
     out, finals = {}, {}
-    for name, kernel in (("companion", "auto"), ("per_step", "naive")):
-        sim = gd.Simulation(nx, ny, nz, kernel=kernel)
+    for name, kernel, blt in (("companion", "auto", 2), ("per_step", "naive", 0)):
+        sim = gd.Simulation(nx, ny, nz, kernel=kernel, blt=blt)
         sim.set_coefficients(W.vacuum_coefficients(SHAPE))
         sim.set_cpml(thickness=L)
         sim.set_sources([dict(component="Jz", wave=wave, i=nx // 2, j=ny // 2, k=nz // 2)])

@@ -15,43 +15,27 @@
 // is the reference's formula, operation for operation, so the interior stays bit-identical to
 // the non-PML solver; psi is stored only in the slabs of its axis (2L + 1 positions).
 //
-// One grid: cpml_e / cpml_h per step, monitors accumulated per step.  A batch of grids:
-// cpml_e_batch / cpml_h_batch cover every grid in one launch each (blockIdx.z = grid * max_nz
-// + k, arguments from a device array) and stage the monitor values for the deferred DFT.
+// Whole grids step with cpml_half<H>: one E and one H launch per step, for one grid or for a
+// group of grids of a batch (blockIdx.z = grid).  Monitor values are staged for the deferred DFT.
+// cpml_region recomputes listed cells for the shell companion of the tiled kernel.
+#include <algorithm>
+
 #include "fdtd_kernels.cuh"
 
 namespace fdtd {
 
 namespace {
 
-struct CoefRefs {
-  const float* c[12];  // pitched per-cell arrays (or null with a material map)
-};
-
-__device__ __forceinline__ void e_coefs(const float* const* A, const uint16_t* mat,
-                                        const Material* tab, long long idx, float* ca, float* cb) {
-  if (mat) {
-    const Material m = tab[mat[idx]];
-    ca[0] = m.a.x; cb[0] = m.a.y; ca[1] = m.a.z; cb[1] = m.a.w; ca[2] = m.b.x; cb[2] = m.b.y;
-  } else {
-    for (int c = 0; c < 3; ++c) {
-      ca[c] = A[c][idx];
-      cb[c] = A[3 + c][idx];
-    }
-  }
+__device__ __forceinline__ void e_coefs(const uint16_t* mat, const Material* tab, long long idx,
+                                        float* ca, float* cb) {
+  const Material m = tab[mat[idx]];
+  ca[0] = m.a.x; cb[0] = m.a.y; ca[1] = m.a.z; cb[1] = m.a.w; ca[2] = m.b.x; cb[2] = m.b.y;
 }
 
-__device__ __forceinline__ void h_coefs(const float* const* A, const uint16_t* mat,
-                                        const Material* tab, long long idx, float* da, float* db) {
-  if (mat) {
-    const Material m = tab[mat[idx]];
-    da[0] = m.b.z; db[0] = m.b.w; da[1] = m.c.x; db[1] = m.c.y; da[2] = m.c.z; db[2] = m.c.w;
-  } else {
-    for (int c = 0; c < 3; ++c) {
-      da[c] = A[6 + c][idx];
-      db[c] = A[9 + c][idx];
-    }
-  }
+__device__ __forceinline__ void h_coefs(const uint16_t* mat, const Material* tab, long long idx,
+                                        float* da, float* db) {
+  const Material m = tab[mat[idx]];
+  da[0] = m.b.z; db[0] = m.b.w; da[1] = m.c.x; db[1] = m.c.y; da[2] = m.c.z; db[2] = m.c.w;
 }
 
 // psi slab element of axis a at slot s for cell (i, j, k)
@@ -86,8 +70,8 @@ __device__ __forceinline__ bool interior(const Grid& g, int i, int j, int k) {
 // E update of interior cell (i, j, k) at step t: E and H of step t from Fi, the new E into Fo
 // (Fi == Fo: in place).
 __device__ __forceinline__ void e_cell(const Grid& g, const FieldPtrs& Fi, const FieldPtrs& Fo,
-                                       const float* const* A, const uint16_t* mat,
-                                       const Material* tab, const Sources& S, long long t,
+                                       const uint16_t* mat, const Material* tab,
+                                       const Sources& S, long long t,
                                        float dx, const CpmlDev& P, int i, int j, int k) {
   const long long sy = g.pitch, sz = g.plane, idx = i + j * sy + k * sz;
   float* const* f = Fi.f;
@@ -120,7 +104,7 @@ __device__ __forceinline__ void e_cell(const Grid& g, const FieldPtrs& Fi, const
     if (src_sum(S, 2, i, j, k, t, &v)) cz = sub(cz, mul(v, dx));
   }
   float ca[3], cb[3];
-  e_coefs(A, mat, tab, idx, ca, cb);
+  e_coefs(mat, tab, idx, ca, cb);
   const float ex = f[0][idx], ey = f[1][idx], ez = f[2][idx];
   Fo.f[0][idx] = yee(ca[0], ex, cb[0], cx);
   Fo.f[1][idx] = yee(ca[1], ey, cb[1], cy);
@@ -130,8 +114,8 @@ __device__ __forceinline__ void e_cell(const Grid& g, const FieldPtrs& Fi, const
 // H update of interior cell (i, j, k) at step t, after every E update of the step: H of step t
 // from Fi, the new E from Fo, the new H into Fo (Fi == Fo: in place).
 __device__ __forceinline__ void h_cell(const Grid& g, const FieldPtrs& Fi, const FieldPtrs& Fo,
-                                       const float* const* A, const uint16_t* mat,
-                                       const Material* tab, const Sources& S, long long t,
+                                       const uint16_t* mat, const Material* tab,
+                                       const Sources& S, long long t,
                                        float dx, const CpmlDev& P, int i, int j, int k) {
   const long long sy = g.pitch, sz = g.plane, idx = i + j * sy + k * sz;
   float* const* f = Fo.f;
@@ -164,62 +148,327 @@ __device__ __forceinline__ void h_cell(const Grid& g, const FieldPtrs& Fi, const
     if (src_sum(S, 5, i, j, k, t, &v)) cz = sub(cz, mul(v, dx));
   }
   float da[3], db[3];
-  h_coefs(A, mat, tab, idx, da, db);
+  h_coefs(mat, tab, idx, da, db);
   const float hx = Fi.f[3][idx], hy = Fi.f[4][idx], hz = Fi.f[5][idx];
   Fo.f[3][idx] = yee(da[0], hx, db[0], cx);
   Fo.f[4][idx] = yee(da[1], hy, db[1], cy);
   Fo.f[5][idx] = yee(da[2], hz, db[2], cz);
 }
 
-// One grid: grid (ceil(nx/32), ceil(ny/4), nz), block (32, 4); interior cells only.
-__global__ void __launch_bounds__(128) cpml_e(Grid g, FieldPtrs F, CoefRefs A, const uint16_t* mat,
-                                              const Material* tab, Sources S, long long t,
-                                              float dx, CpmlDev P) {
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y, k = blockIdx.z;
-  if (interior(g, i, j, k)) e_cell(g, F, F, A.c, mat, tab, S, t, dx, P, i, j, k);
+// ------------------------------------------------------------------ whole-grid half steps
+// A thread owns kCpmlV = 2 consecutive x cells (a cell pair, one 8-byte access per field) of one
+// row and marches along z, so the z-neighbours of the curls are its own registers of the plane
+// before and everything that depends on x and y alone (addresses, layer slots and profiles of x
+// and y, face tests) is computed once per march instead of once per cell.  The pairs of a row
+// that touch an x layer (XL) are marched by blocks of their own: no warp runs the x-layer code
+// for a few of its lanes.  The y layers are uniform along a row, the z layers along a plane.
+//
+// Bound: memory latency at the occupancy the registers allow (38 bytes per cell and half step
+// plus the layers' psi).  So all loads of a plane are issued before its first store (a psi load
+// behind another psi array's store would wait for it), and the pointers stay in the constant
+// bank (kernel parameters) instead of registers.  B200, both half steps: 32 grids of 96^3 with 8
+// layer cells 0.61 ms a step (46 Gcell-updates/s; one thread per cell without a march 1.57 ms),
+// 256^3 with 10 layer cells 0.30 ms (55 Gcell-updates/s; 0.52 ms).  Four cells per thread (128
+// registers, 12 warps per SM instead of 20) took 0.74 ms and 0.33 ms.  Stepping the batch group
+// by group, each group small enough for the L2 cache, took longer (0.69 ms): what is missing
+// are loads in flight, not bandwidth.
+constexpr int V = kCpmlV;
+constexpr int kHalfThreads = 128;
+
+struct Cells {
+  float v[V];
+};
+__device__ __forceinline__ Cells ldv(const float* p) {
+  const float2 f = *reinterpret_cast<const float2*>(p);
+  return {{f.x, f.y}};
+}
+__device__ __forceinline__ void stv(float* p, const Cells& q) {
+  *reinterpret_cast<float2*>(p) = make_float2(q.v[0], q.v[1]);
+}
+__device__ __forceinline__ Cells subv(const Cells& a, const Cells& b) {
+  Cells r;
+#pragma unroll
+  for (int e = 0; e < V; ++e) r.v[e] = sub(a.v[e], b.v[e]);
+  return r;
 }
 
-__global__ void __launch_bounds__(128) cpml_h(Grid g, FieldPtrs F, CoefRefs A, const uint16_t* mat,
-                                              const Material* tab, Sources S, long long t,
-                                              float dx, CpmlDev P) {
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y, k = blockIdx.z;
-  if (interior(g, i, j, k)) h_cell(g, F, F, A.c, mat, tab, S, t, dx, P, i, j, k);
+// psi of V cells of one row along y or z; vec: whole-pair accesses are aligned.  Cells outside
+// `upd` (faces, padding) have no psi.
+__device__ __forceinline__ Cells ld_psi(const float* psi, bool vec, const bool* upd) {
+  if (vec) return ldv(psi);
+  Cells p;
+#pragma unroll
+  for (int e = 0; e < V; ++e) p.v[e] = upd[e] ? psi[e] : 0.0f;
+  return p;
 }
-
-// Monitor values of cell (i, j) of plane k at step t into the staging rings: the E monitors
-// after the E update (e_comps), the H monitors after the H update.  Face cells, which the update
-// leaves unchanged, are staged too: the fold reads every cell of the plane.
-__device__ __forceinline__ void stage_cell(const CpmlSim& s, long long t, int i, int j, int k,
-                                           bool e_comps) {
-  for (int n = 0; n < s.M.n; ++n) {
-    const MonitorDev& m = s.M.m[n];
-    if ((m.comp < 3) != e_comps || m.k != k) continue;
-    const long long idx = i + (long long)j * s.g.pitch + (long long)k * s.g.plane;
-    dft_record(m, t, i, j, s.g, s.F.f[m.comp][idx]);
+__device__ __forceinline__ void st_psi(float* psi, const Cells& p, bool vec, const bool* upd) {
+  if (vec) {
+    stv(psi, p);
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < V; ++e)
+    if (upd[e]) psi[e] = p.v[e];
+}
+// d <- d / kappa + psi for one profile entry; p becomes the new psi in the cells of `upd`.
+__device__ __forceinline__ void stretch(Cells& d, float b, float a, float ik, Cells& p,
+                                        const bool* upd) {
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const float n = add(mul(b, p.v[e]), mul(a, d.v[e]));
+    p.v[e] = upd[e] ? n : p.v[e];
+    d.v[e] = add(mul(d.v[e], ik), n);
   }
 }
 
-// A batch: blockIdx.z = grid * max_nz + k over the grids' argument array.
-__global__ void __launch_bounds__(128) cpml_e_batch(const CpmlSim* sims, int max_nz,
-                                                    long long t_offset) {
-  const CpmlSim& s = sims[blockIdx.z / max_nz];
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
-  const int k = (int)(blockIdx.z % max_nz);
-  if (i >= s.g.nx || j >= s.g.ny || k >= s.g.nz) return;
-  const long long t = s.t0 + t_offset;
-  if (interior(s.g, i, j, k)) e_cell(s.g, s.F, s.F, s.coef, s.mat, s.tab, s.S, t, s.dx, s.P, i, j, k);
-  if (s.M.n) stage_cell(s, t, i, j, k, true);
+// E (H = false) or H half step of step t over planes [k0, k1) of cells i0 .. i0+V-1 of row j, in
+// place.  P: layers; s: sources, monitors, material and per-cell coefficients.
+template <bool H, bool XL>
+__device__ __forceinline__ void march_row(const CpmlHot& h, const CpmlSim& s, long long t, int i0,
+                                          int j, int k0, int k1) {
+  const Grid& g = h.g;
+  const bool jrow = j >= 1 && j <= g.ny - 2;
+  bool upd[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) upd[e] = jrow && i0 + e >= 1 && i0 + e <= g.nx - 2;
+  const bool vec = (g.nx & (V - 1)) == 0;
+  const CpmlAxis &X = h.P.ax[0], &Y = h.P.ax[1], &Z = h.P.ax[2];
+  // x layers: a layer's slots are consecutive, xs + e for the cells with xin[e]
+  int xs = 0;
+  bool xin[V] = {};
+  float xb[V], xa[V], xi[V];
+  if (XL) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const int i = min(i0 + e, g.nx - 1), sl = H ? X.slot_h[i] : X.slot_e[i];
+      xin[e] = upd[e] && sl >= 0;
+      if (xin[e]) xs = sl - e;
+      xb[e] = H ? X.bh[i] : X.be[i];
+      xa[e] = H ? X.ah[i] : X.ae[i];
+      xi[e] = H ? X.ikh[i] : X.ike[i];
+    }
+  }
+  const int ys = H ? Y.slot_h[j] : Y.slot_e[j];
+  const float yb = H ? Y.bh[j] : Y.be[j], ya = H ? Y.ah[j] : Y.ae[j], yi = H ? Y.ikh[j] : Y.ike[j];
+  const int lean_id = s.lean ? s.lean_id : -1;
+  const float lean_c = H ? s.lean_db : s.lean_cb;
+  // planes that some source or monitor of this half step touches
+  int slo = 1 << 30, shi = -1, mlo = 1 << 30, mhi = -1;
+  for (int n = 0; n < s.S.n; ++n)
+    if ((s.S.s[n].comp >= 3) == H) slo = min(slo, s.S.s[n].k), shi = max(shi, s.S.s[n].k);
+  for (int n = 0; n < s.M.n; ++n)
+    if ((s.M.m[n].comp >= 3) == H) mlo = min(mlo, s.M.m[n].k), mhi = max(mhi, s.M.m[n].k);
+
+  // offset of the row's cells in a plane; the planes' bases are uniform
+  const uint32_t o = (uint32_t)(i0 + j * g.pitch);
+  const uint32_t oy = H ? o + (uint32_t)g.pitch : o - (uint32_t)g.pitch;
+  // E: components 0, 1 of H at plane k-1; H: components 0, 1 of E at plane k
+  Cells c0 = {}, c1 = {};
+  if (jrow && k0 + (H ? 0 : -1) >= 0) {
+    const long long b = (long long)(k0 + (H ? 0 : -1)) * g.plane;
+    c0 = ldv(h.F.f[H ? 0 : 3] + b + o);
+    c1 = ldv(h.F.f[H ? 1 : 4] + b + o);
+  }
+  for (int k = k0; k < k1; ++k) {
+    const long long base = (long long)k * g.plane;
+    const long long bnew = base + (H ? g.plane : 0);
+    // fields differenced (s0, s1, s2) and advanced (d0, d1, d2)
+    const float* const s0 = h.F.f[H ? 0 : 3] + base;
+    const float* const s1 = h.F.f[H ? 1 : 4] + base;
+    const float* const s2 = h.F.f[H ? 2 : 5] + base;
+    const float* const n0p = h.F.f[H ? 0 : 3] + bnew;
+    const float* const n1p = h.F.f[H ? 1 : 4] + bnew;
+    float* const d0 = h.F.f[H ? 3 : 0] + base;
+    float* const d1 = h.F.f[H ? 4 : 1] + base;
+    float* const d2 = h.F.f[H ? 5 : 2] + base;
+    if (jrow) {
+      if (k >= 1 && k <= g.nz - 2) {
+        // Every load of the plane first: a psi load behind the store of another psi array would
+        // wait for it (they may alias as far as the compiler knows), one memory latency each.
+        Cells f0 = ldv(d0 + o), f1 = ldv(d1 + o), f2 = ldv(d2 + o);
+        const Cells v2 = ldv(s2 + o);
+        const Cells n0 = ldv(n0p + o), n1 = ldv(n1p + o);
+        const Cells y0 = ldv(s0 + oy), y2 = ldv(s2 + oy);
+        float x1 = 0.0f, x2 = 0.0f;
+        if (H ? i0 + V < g.nx : i0 > 0) {
+          x1 = s1[o + (H ? V : -1)];
+          x2 = s2[o + (H ? V : -1)];
+        }
+        ushort2 id = {};
+        if (h.mat) id = *reinterpret_cast<const ushort2*>(h.mat + base + o);
+        const int zs = H ? Z.slot_h[k] : Z.slot_e[k];
+        Cells py2, py0, pz1, pz0;
+        Cells px2, px1;
+        const uint32_t oyp = (uint32_t)(i0 + g.nx * ys), ozp = (uint32_t)(i0 + g.nx * j);
+        const long long byp = (long long)g.nx * Y.S * k, bzp = (long long)g.nx * g.ny * zs;
+        const uint32_t oxp = (uint32_t)(xs + X.S * j);
+        const long long bxp = (long long)X.S * g.ny * k;
+        float* const* psi = H ? h.P.psi_h : h.P.psi_e;
+        if (ys >= 0) {
+          py2 = ld_psi(psi[H ? 1 : 0] + byp + oyp, vec, upd);
+          py0 = ld_psi(psi[H ? 4 : 5] + byp + oyp, vec, upd);
+        }
+        if (zs >= 0) {
+          pz1 = ld_psi(psi[H ? 0 : 1] + bzp + ozp, vec, upd);
+          pz0 = ld_psi(psi[H ? 3 : 2] + bzp + ozp, vec, upd);
+        }
+        if (XL) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            px2.v[e] = xin[e] ? psi[H ? 2 : 3][bxp + oxp + e] : 0.0f;
+            px1.v[e] = xin[e] ? psi[H ? 5 : 4][bxp + oxp + e] : 0.0f;
+          }
+        }
+        // curl = (dy2 - dz1, dz0 - dx2, dx1 - dy0) for E, the negative for H
+        Cells dy2 = H ? subv(y2, v2) : subv(v2, y2), dy0 = H ? subv(y0, c0) : subv(n0, y0);
+        Cells dz1 = subv(n1, c1), dz0 = subv(n0, c0), dx2, dx1;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          if (!H) {
+            dx2.v[e] = sub(v2.v[e], e ? v2.v[e - 1] : x2);
+            dx1.v[e] = sub(n1.v[e], e ? n1.v[e - 1] : x1);
+          } else {
+            dx2.v[e] = sub(e < V - 1 ? v2.v[e + 1] : x2, v2.v[e]);
+            dx1.v[e] = sub(e < V - 1 ? c1.v[e + 1] : x1, c1.v[e]);
+          }
+        }
+        if (ys >= 0) {
+          stretch(dy2, yb, ya, yi, py2, upd);
+          stretch(dy0, yb, ya, yi, py0, upd);
+          st_psi(psi[H ? 1 : 0] + byp + oyp, py2, vec, upd);
+          st_psi(psi[H ? 4 : 5] + byp + oyp, py0, vec, upd);
+        }
+        if (zs >= 0) {
+          const float b = H ? Z.bh[k] : Z.be[k], a = H ? Z.ah[k] : Z.ae[k];
+          const float ik = H ? Z.ikh[k] : Z.ike[k];
+          stretch(dz1, b, a, ik, pz1, upd);
+          stretch(dz0, b, a, ik, pz0, upd);
+          st_psi(psi[H ? 0 : 1] + bzp + ozp, pz1, vec, upd);
+          st_psi(psi[H ? 3 : 2] + bzp + ozp, pz0, vec, upd);
+        }
+        if (XL) {
+#pragma unroll
+          for (int e = 0; e < V; ++e)
+            if (xin[e]) {
+              px2.v[e] = add(mul(xb[e], px2.v[e]), mul(xa[e], dx2.v[e]));
+              px1.v[e] = add(mul(xb[e], px1.v[e]), mul(xa[e], dx1.v[e]));
+              dx2.v[e] = add(mul(dx2.v[e], xi[e]), px2.v[e]);
+              dx1.v[e] = add(mul(dx1.v[e], xi[e]), px1.v[e]);
+              psi[H ? 2 : 3][bxp + oxp + e] = px2.v[e];
+              psi[H ? 5 : 4][bxp + oxp + e] = px1.v[e];
+            }
+        }
+        // E: (dyHz - dzHy, dzHx - dxHz, dxHy - dyHx); H: (dzEy - dyEz, dxEz - dzEx, dyEx - dxEy)
+        Cells u0 = H ? subv(dz1, dy2) : subv(dy2, dz1);
+        Cells u1 = H ? subv(dx2, dz0) : subv(dz0, dx2);
+        Cells u2 = H ? subv(dy0, dx1) : subv(dx1, dy0);
+        if (k >= slo && k <= shi) {
+          const float dx = s.dx;
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            float v;
+            if (source_value(s.S, H ? 3 : 0, i0 + e, j, k, t, &v)) u0.v[e] = sub(u0.v[e], mul(v, dx));
+            if (source_value(s.S, H ? 4 : 1, i0 + e, j, k, t, &v)) u1.v[e] = sub(u1.v[e], mul(v, dx));
+            if (source_value(s.S, H ? 5 : 2, i0 + e, j, k, t, &v)) u2.v[e] = sub(u2.v[e], mul(v, dx));
+          }
+        }
+        if (h.mat) {
+          const int ids[V] = {id.x, id.y};
+          if (id.x == lean_id && id.y == lean_id) {
+#pragma unroll
+            for (int e = 0; e < V; ++e) {  // the a coefficients are 1 and 1 * f == f
+              f0.v[e] = upd[e] ? add(f0.v[e], mul(lean_c, u0.v[e])) : f0.v[e];
+              f1.v[e] = upd[e] ? add(f1.v[e], mul(lean_c, u1.v[e])) : f1.v[e];
+              f2.v[e] = upd[e] ? add(f2.v[e], mul(lean_c, u2.v[e])) : f2.v[e];
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+              const Material* m = h.tab + ids[e];
+              const float2 q = __ldg(reinterpret_cast<const float2*>(&m->b) + (H ? 1 : 0));
+              const float4 w = __ldg(H ? &m->c : &m->a);
+              // E: {Cax, Cbx, Cay, Cby} = w, {Caz, Cbz} = q; H: {Dax, Dbx} = q, {Day .. Dbz} = w
+              const float m0 = H ? yee(q.x, f0.v[e], q.y, u0.v[e]) : yee(w.x, f0.v[e], w.y, u0.v[e]);
+              const float m1 = H ? yee(w.x, f1.v[e], w.y, u1.v[e]) : yee(w.z, f1.v[e], w.w, u1.v[e]);
+              const float m2 = H ? yee(w.z, f2.v[e], w.w, u2.v[e]) : yee(q.x, f2.v[e], q.y, u2.v[e]);
+              f0.v[e] = upd[e] ? m0 : f0.v[e];
+              f1.v[e] = upd[e] ? m1 : f1.v[e];
+              f2.v[e] = upd[e] ? m2 : f2.v[e];
+            }
+          }
+        } else {
+          const int c = H ? 6 : 0;
+          const Cells a0 = ldv(s.coef[c] + base + o), b0 = ldv(s.coef[c + 3] + base + o);
+          const Cells a1 = ldv(s.coef[c + 1] + base + o), b1 = ldv(s.coef[c + 4] + base + o);
+          const Cells a2 = ldv(s.coef[c + 2] + base + o), b2 = ldv(s.coef[c + 5] + base + o);
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            f0.v[e] = upd[e] ? yee(a0.v[e], f0.v[e], b0.v[e], u0.v[e]) : f0.v[e];
+            f1.v[e] = upd[e] ? yee(a1.v[e], f1.v[e], b1.v[e], u1.v[e]) : f1.v[e];
+            f2.v[e] = upd[e] ? yee(a2.v[e], f2.v[e], b2.v[e], u2.v[e]) : f2.v[e];
+          }
+        }
+        stv(d0 + o, f0);
+        stv(d1 + o, f1);
+        stv(d2 + o, f2);
+        c0 = n0;
+        c1 = n1;
+      } else if (k + (H ? 1 : 0) < g.nz) {  // a z face: nothing changes, carry the neighbours on
+        c0 = ldv(n0p + o);
+        c1 = ldv(n1p + o);
+      }
+    }
+    if (k >= mlo && k <= mhi) {  // face cells too: the fold reads every cell of the plane
+      for (int n = 0; n < s.M.n; ++n) {
+        const MonitorDev& m = s.M.m[n];
+        if ((m.comp >= 3) != H || m.k != k) continue;
+        const float* f = h.F.f[m.comp] + base + o;
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (i0 + e < g.nx) dft_record(m, t, i0 + e, j, g, f[e]);
+      }
+    }
+  }
 }
 
-__global__ void __launch_bounds__(128) cpml_h_batch(const CpmlSim* sims, int max_nz,
-                                                    long long t_offset) {
-  const CpmlSim& s = sims[blockIdx.z / max_nz];
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
-  const int k = (int)(blockIdx.z % max_nz);
-  if (i >= s.g.nx || j >= s.g.ny || k >= s.g.nz) return;
-  const long long t = s.t0 + t_offset;
-  if (interior(s.g, i, j, k)) h_cell(s.g, s.F, s.F, s.coef, s.mat, s.tab, s.S, t, s.dx, s.P, i, j, k);
-  if (s.M.n) stage_cell(s, t, i, j, k, false);
+// Work of CTA b of the blocks of one z-chunk: first the quads off the x layers, then those that
+// touch one.
+template <bool H>
+__device__ __forceinline__ void half_block(const CpmlHot& h, const CpmlSim& s, long long t, int b,
+                                           int k0, int k1) {
+  const Grid& g = h.g;
+  const int nq = (g.nx + V - 1) / V, nl = h.ql[H], nlay = nl + h.qr[H], nint = nq - nlay;
+  const int bint = (nint * g.ny + kHalfThreads - 1) / kHalfThreads;
+  if (b < bint) {
+    const int q = b * kHalfThreads + (int)threadIdx.x;
+    const int j = q / nint;
+    if (j < g.ny) march_row<H, false>(h, s, t, V * (nl + q - j * nint), j, k0, k1);
+  } else if (nlay > 0) {
+    const int q = (b - bint) * kHalfThreads + (int)threadIdx.x;
+    const int j = q / nlay, l = q - j * nlay;
+    if (j < g.ny) march_row<H, true>(h, s, t, V * (l < nl ? l : l + nint), j, k0, k1);
+  }
+}
+
+// One grid (arguments in the parameters): blockIdx.x = cells, blockIdx.y = z-chunk of zc planes.
+template <bool H>
+__global__ void __launch_bounds__(kHalfThreads, 6) cpml_half(const __grid_constant__ CpmlHot h,
+                                                          const __grid_constant__ CpmlSim s,
+                                                          long long t, int zc) {
+  const int k0 = (int)blockIdx.y * zc;
+  half_block<H>(h, s, t, (int)blockIdx.x, k0, min(h.g.nz, k0 + zc));
+}
+
+// A group of grids of a batch: blockIdx.z = grid of the group.
+template <bool H>
+__global__ void __launch_bounds__(kHalfThreads, 6)
+    cpml_half_batch(const __grid_constant__ CpmlGroup grp, const CpmlSim* __restrict__ sims,
+                    long long t_offset, int zc) {
+  const CpmlHot& h = grp.h[blockIdx.z];
+  const CpmlSim& s = sims[blockIdx.z];
+  const int k0 = (int)blockIdx.y * zc;
+  if (k0 >= h.g.nz) return;
+  half_block<H>(h, s, s.t0 + t_offset, (int)blockIdx.x, k0, min(h.g.nz, k0 + zc));
 }
 
 // The shell companion: blockIdx.x indexes the block list; cells inside `inner` return.
@@ -238,9 +487,9 @@ __global__ void __launch_bounds__(128) cpml_region(Grid g, FieldPtrs Fi, FieldPt
   const int c0 = H ? 3 : 0;
   if (interior(g, i, j, k)) {
     if (H)
-      h_cell(g, Fi, Fo, nullptr, mat, tab, S, t, dx, P, i, j, k);
+      h_cell(g, Fi, Fo, mat, tab, S, t, dx, P, i, j, k);
     else
-      e_cell(g, Fi, Fo, nullptr, mat, tab, S, t, dx, P, i, j, k);
+      e_cell(g, Fi, Fo, mat, tab, S, t, dx, P, i, j, k);
   } else if (Fi.f[c0] != Fo.f[c0]) {  // faces never change: carry them into the output set
     for (int c = c0; c < c0 + 3; ++c) Fo.f[c][idx] = Fi.f[c][idx];
   }
@@ -268,36 +517,57 @@ cudaError_t launch_cpml_region(bool h_half, const Grid& g, const FieldPtrs& Fi,
   return cudaGetLastError();
 }
 
-cudaError_t launch_cpml_batch_step(const CpmlSim* sims, int nsims, int max_nx, int max_ny,
-                                   int max_nz, long long t_offset, cudaStream_t st) {
-  if (nsims <= 0) return cudaSuccess;
-  if (max_nz <= 0 || max_nz > 65535) return cudaErrorInvalidValue;
-  // grids per launch pair: blockIdx.z stays within its 65535 limit (grids are independent, so
-  // each group's E launch before its H launch is all the order a step needs)
-  const int per = 65535 / max_nz;
-  const dim3 blk(32, 4);
-  for (int g0 = 0; g0 < nsims; g0 += per) {
-    const int n = nsims - g0 < per ? nsims - g0 : per;
-    const dim3 grd((max_nx + 31) / 32, (max_ny + 3) / 4, (unsigned)(n * max_nz));
-    cpml_e_batch<<<grd, blk, 0, st>>>(sims + g0, max_nz, t_offset);
-    cpml_h_batch<<<grd, blk, 0, st>>>(sims + g0, max_nz, t_offset);
+namespace {
+
+// Blocks that cover one z-chunk of grid h (the more of the E and the H half step).
+int cpml_blocks(const CpmlHot& h) {
+  int most = 0;
+  for (int k = 0; k < 2; ++k) {
+    const int nlay = h.ql[k] + h.qr[k], nint = (h.g.nx + V - 1) / V - nlay;
+    most = std::max(most, (nint * h.g.ny + kHalfThreads - 1) / kHalfThreads +
+                              (nlay * h.g.ny + kHalfThreads - 1) / kHalfThreads);
   }
+  return most;
+}
+
+// Planes per z-chunk: a longer march amortises its set-up and the extra plane it loads, but
+// every SM should have several blocks.
+int cpml_planes(long long blocks, int nz) {
+  int zc = 16;
+  while (zc > 4 && blocks * ((nz + zc - 1) / zc) < 148 * 8) zc /= 2;
+  return zc;
+}
+
+}  // namespace
+
+cudaError_t launch_cpml_batch_step(const CpmlGroup& grp, int n, const CpmlSim* sims,
+                                   long long t_offset, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  if (n > kCpmlGroup) return cudaErrorInvalidValue;
+  long long blocks = 0;
+  int most = 0, max_nz = 0;
+  for (int q = 0; q < n; ++q) {
+    const int b = cpml_blocks(grp.h[q]);
+    blocks += b;
+    most = std::max(most, b);
+    max_nz = std::max(max_nz, grp.h[q].g.nz);
+  }
+  const int zc = std::max(cpml_planes(blocks, max_nz), (max_nz + 65534) / 65535);
+  const dim3 grd((unsigned)most, (unsigned)((max_nz + zc - 1) / zc), (unsigned)n);
+  cpml_half_batch<false><<<grd, kHalfThreads, 0, st>>>(grp, sims, t_offset, zc);
+  cpml_half_batch<true><<<grd, kHalfThreads, 0, st>>>(grp, sims, t_offset, zc);
   return cudaGetLastError();
 }
 
-cudaError_t launch_cpml_step(const Grid& g, const FieldPtrs& F, const float* const* coef,
-                             const uint16_t* mat, const Material* tab, const Sources& S,
-                             const Monitors& M, const CpmlDev& P, long long t, float dx,
-                             cudaStream_t st, int* launches) {
-  CoefRefs A;
-  for (int c = 0; c < 12; ++c) A.c[c] = coef ? coef[c] : nullptr;
-  const dim3 blk(32, 4), grd((g.nx + 31) / 32, (g.ny + 3) / 4, g.nz);
-  cpml_e<<<grd, blk, 0, st>>>(g, F, A, mat, tab, S, t, dx, P);
-  cpml_h<<<grd, blk, 0, st>>>(g, F, A, mat, tab, S, t, dx, P);
+cudaError_t launch_cpml_step(const CpmlHot& h, const CpmlSim& s, long long t, cudaStream_t st,
+                             int* launches) {
+  const int nb = cpml_blocks(h);
+  const int zc = std::max(cpml_planes(nb, h.g.nz), (h.g.nz + 65534) / 65535);
+  const dim3 grd((unsigned)nb, (unsigned)((h.g.nz + zc - 1) / zc));
+  cpml_half<false><<<grd, kHalfThreads, 0, st>>>(h, s, t, zc);
+  cpml_half<true><<<grd, kHalfThreads, 0, st>>>(h, s, t, zc);
   *launches += 2;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || M.n == 0) return e;
-  return launch_naive_dft(g, F, M, t, st, launches);
+  return cudaGetLastError();
 }
 
 }  // namespace fdtd

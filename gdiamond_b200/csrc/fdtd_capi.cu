@@ -125,6 +125,7 @@ struct fdtd_handle {
   std::vector<int> cpml_slot[3][2];      // host copies of the slot tables (E, H positions)
   std::vector<float> cpml_prof[3][2][3]; // host copies of b, a, 1/kappa
   fdtd::CpmlDev cpml_dev{};
+  int cpml_groups[2][2] = {};  // E, H positions: cell groups of a row in the lower / upper x layer
   // Shell companion of the tiled kernel (cpml_companion): cpml_inner = per axis the [lo, hi)
   // range of positions whose E and H updates involve no layer, cpml_lo / cpml_hi = the axis has
   // a layer on that side; a third FP32 field set for the companion's intermediate steps; block
@@ -399,17 +400,7 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
       return FDTD_OK;
     }
   }
-  std::vector<fdtd::TiledConfig> cands = candidates(h);
-  if (h->cpml_on) {
-    // With CPML layers the shell companion recomputes regions about 3 BLT cells deeper than
-    // the layers after every launch, so its cost grows with BLT while the timing below sees the
-    // tiled kernel alone: keep BLT <= 2 (by estimate the best total at 256^3 with 10-cell
-    // layers; BLT 6 measured slower overall).
-    std::vector<fdtd::TiledConfig> keep;
-    for (const auto& c : cands)
-      if (c.blt <= 2) keep.push_back(c);
-    if (!keep.empty()) cands.swap(keep);
-  }
+  const std::vector<fdtd::TiledConfig> cands = candidates(h);
   if (cands.empty()) return fail(h, FDTD_ERR_UNSUPPORTED, "no tiled configuration fits this grid");
   if (cands.size() == 1) {
     h->cfg = cands[0];
@@ -895,6 +886,41 @@ fdtd_status cpml_companion(fdtd_handle* h, int k, int src, int dst, long long t,
   return FDTD_OK;
 }
 
+// Kernel arguments of handle h's whole-grid CPML steps.
+fdtd::CpmlHot make_cpml_hot(const fdtd_handle* h) {
+  fdtd::CpmlHot a;
+  memset(&a, 0, sizeof(a));  // compared bytewise (graph key)
+  a.g = h->g;
+  for (int c = 0; c < 6; ++c) a.F.f[c] = h->F[h->cur][c];
+  if (h->coef_mode == kCoefMaterial) {
+    a.mat = h->mat;
+    a.tab = h->table;
+  }
+  a.P = h->cpml_dev;
+  for (int k = 0; k < 2; ++k) {
+    a.ql[k] = h->cpml_groups[k][0];
+    a.qr[k] = h->cpml_groups[k][1];
+  }
+  return a;
+}
+fdtd::CpmlSim make_cpml_sim(const fdtd_handle* h) {
+  fdtd::CpmlSim a{};
+  a.g = h->g;
+  if (h->coef_mode == kCoefMaterial) {
+    a.lean = h->lean_ok && h->lean_enable ? 1 : 0;
+    a.lean_id = h->lean_id;
+    a.lean_cb = h->lean_cb;
+    a.lean_db = h->lean_db;
+  } else {
+    for (int c = 0; c < 12; ++c) a.coef[c] = h->coef[c];
+  }
+  a.S = make_sources(h);
+  a.M = make_monitors(h);
+  a.t0 = h->t;
+  a.dx = h->desc.dx;
+  return a;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1219,35 +1245,40 @@ fdtd_status fdtd_step(fdtd_handle* h, int64_t T, void* stream) {
   }
   fdtd_status s = ensure_tables(h, h->t + T);
   if (s != FDTD_OK) return s;
-  // CPML layers: the tiled kernel with the shell companion when the grid is large enough for
-  // it (and the caller did not ask for the naive kernel), else one E and one H kernel per step
-  // over the whole grid, monitors per step.
+  // CPML layers: one E and one H kernel per step over the whole grid, monitors staged; or, when
+  // the caller asks for a temporal block (desc.blt) and the grid is large enough for it, the tiled
+  // kernel with the shell companion.  The companion recomputes a third of a 256^3 grid with
+  // 10-cell layers and was the slower of the two there (0.45 against 0.30 ms a step).
   bool companion = false;
   if (h->cpml_on) {
     if (h->storage != FDTD_STORE_F32)
       return fail(h, FDTD_ERR_UNSUPPORTED, "CPML layers need FP32 field storage");
-    if (h->desc.kernel != FDTD_KERNEL_NAIVE && h->coef_mode == kCoefMaterial &&
-        cpml_companion_fits(h, 1)) {
+    if (h->desc.kernel != FDTD_KERNEL_NAIVE && h->desc.blt > 0 &&
+        h->coef_mode == kCoefMaterial && cpml_companion_fits(h, 1)) {
       if (!h->cfg_ready && (s = autotune(h, st)) != FDTD_OK) return s;
       companion = cpml_companion_fits(h, h->cfg.blt);
     }
   }
   if (h->cpml_on && !companion) {
-    fdtd::FieldPtrs F;
-    for (int c = 0; c < 6; ++c) F.f[c] = h->F[h->cur][c];
-    const bool matm = h->coef_mode == kCoefMaterial;
-    const fdtd::Sources S = make_sources(h);
-    const fdtd::Monitors M = make_monitors(h);
-    int launches = 0;
+    const fdtd::CpmlSim sim = make_cpml_sim(h);
+    const fdtd::CpmlHot hot = make_cpml_hot(h);
+    int launches = 0, folds = 0;
+    long long t_fold = h->t;
+    auto fold = [&]() -> fdtd_status {
+      CUDA_TRY(h, fdtd::launch_dft_fold(sim.M, h->g, t_fold, (int)(h->t - t_fold), st));
+      ++folds;
+      t_fold = h->t;
+      return FDTD_OK;
+    };
     for (int64_t q = 0; q < T; ++q) {
-      CUDA_TRY(h, fdtd::launch_cpml_step(h->g, F, matm ? nullptr : h->coef,
-                                         matm ? h->mat : nullptr, h->table, S, M, h->cpml_dev,
-                                         h->t, h->desc.dx, st, &launches));
+      if (sim.M.n > 0 && h->t + 1 - t_fold > fdtd::kDftSlots && (s = fold()) != FDTD_OK) return s;
+      CUDA_TRY(h, fdtd::launch_cpml_step(hot, sim, h->t, st, &launches));
       h->t += 1;
     }
+    if (sim.M.n > 0 && h->t > t_fold && (s = fold()) != FDTD_OK) return s;
     h->last_kernel = 6;  // reported by fdtd_get_config: the per-step CPML kernels
     h->last_launches = launches;
-    h->last_folds = 0;
+    h->last_folds = folds;
     if (st != h->stream) {
       cudaEvent_t ev;
       CUDA_TRY(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -1624,6 +1655,20 @@ fdtd_status fdtd_set_cpml(fdtd_handle* h, const fdtd_cpml_desc* d) {
     h->cpml_lo[a] = lo > 0;
     h->cpml_hi[a] = hi < n[a];
   }
+  for (int k = 0; k < 2; ++k) {
+    const std::vector<int>& sl = h->cpml_slot[0][k];
+    constexpr int V = fdtd::kCpmlV;
+    const int nq = (n[0] + V - 1) / V;
+    int ql = 0, qr = 0;
+    for (int p = 0; p < n[0]; ++p) {
+      if (sl[p] < 0) continue;
+      if (2 * p < n[0]) ql = std::max(ql, p / V + 1);
+      else qr = std::max(qr, nq - p / V);
+    }
+    if (ql + qr > nq) ql = nq, qr = 0;  // a group of both layers
+    h->cpml_groups[k][0] = ql;
+    h->cpml_groups[k][1] = qr;
+  }
   h->cpml_on = true;
   return FDTD_OK;
 }
@@ -1930,67 +1975,64 @@ fdtd_status stream_after(fdtd_batch* b, cudaStream_t waiter, cudaStream_t on) {
   return FDTD_OK;
 }
 
-// A batch whose simulations have CPML layers: per step one E and one H launch over every grid
-// (in place, FP32), monitor values staged in the rings and folded before a ring would wrap and
-// at the end, as in the tiled batches.  With use_graph the T steps are captured once and
-// replayed; the argument table is refreshed by the copy at the head of the sequence, so the
-// graph only depends on T and the batch's extents.
+// A batch whose simulations have CPML layers: per step one E and one H launch over up to
+// kCpmlGroup grids (in place, FP32), monitor values staged in the rings and folded before a ring
+// would wrap and at the end, as in the tiled batches.  With use_graph the T steps are captured
+// once and replayed; what changes from call to call (step counters, sources, monitors, materials)
+// is in the argument table refreshed by the copy at the head of the sequence, the rest (CpmlHot)
+// is in the graph's key.
 fdtd_status batch_step_cpml(fdtd_batch* b, int64_t T, int32_t use_graph, cudaStream_t st) {
   const int n = (int)b->sims.size();
   if (!b->h_cpml) {
     BCUDA(b, cudaMalloc(&b->d_cpml, n * sizeof(fdtd::CpmlSim)));
     BCUDA(b, cudaMallocHost(&b->h_cpml, n * sizeof(fdtd::CpmlSim)));
   }
-  int max_nx = 0, max_ny = 0, max_nz = 0, max_nf = 0;
+  int max_nf = 0;
   long long max_np = 0;
+  std::vector<fdtd::CpmlHot> hot(n);
   for (int i = 0; i < n; ++i) {
     const fdtd_handle* h = b->sims[i];
     if (h->storage != FDTD_STORE_F32)
       return bfail(b, FDTD_ERR_UNSUPPORTED, "CPML layers need FP32 field storage");
-    fdtd::CpmlSim& a = b->h_cpml[i];
-    a = fdtd::CpmlSim{};
-    a.g = h->g;
-    for (int c = 0; c < 6; ++c) a.F.f[c] = h->F[h->cur][c];
-    a.mat = h->mat;  // batches hold material maps only
-    a.tab = h->table;
-    a.S = make_sources(h);
-    a.M = make_monitors(h);
-    a.P = h->cpml_dev;
-    a.t0 = h->t;
-    a.dx = h->desc.dx;
-    max_nx = std::max(max_nx, h->g.nx);
-    max_ny = std::max(max_ny, h->g.ny);
-    max_nz = std::max(max_nz, h->g.nz);
+    b->h_cpml[i] = make_cpml_sim(h);
+    hot[i] = make_cpml_hot(h);
     for (int m = 0; m < h->nmon; ++m) {
       max_np = std::max<long long>(max_np, (long long)h->g.nx * h->g.ny);
       max_nf = std::max(max_nf, h->mon[m].nf);
     }
   }
+  const int ngroups = (n + fdtd::kCpmlGroup - 1) / fdtd::kCpmlGroup;
   int folds = 0;
   auto record = [&](cudaStream_t rs) -> fdtd_status {
     BCUDA(b, cudaMemcpyAsync(b->d_cpml, b->h_cpml, n * sizeof(fdtd::CpmlSim),
                              cudaMemcpyHostToDevice, rs));
     long long folded = 0;
     folds = 0;
-    for (long long q = 0; q < T; ++q) {
-      if (max_nf > 0 && q + 1 - folded > fdtd::kDftSlots) {
+    for (long long q = 0; q <= T; ++q) {
+      if (max_nf > 0 && q > folded && (q == T || q + 1 - folded > fdtd::kDftSlots)) {
         BCUDA(b, fdtd::launch_dft_fold_cpml_batch(b->d_cpml, n, max_np, max_nf, folded,
                                                   (int)(q - folded), rs));
         ++folds;
         folded = q;
       }
-      BCUDA(b, fdtd::launch_cpml_batch_step(b->d_cpml, n, max_nx, max_ny, max_nz, q, rs));
-    }
-    if (max_nf > 0 && T > folded) {
-      BCUDA(b, fdtd::launch_dft_fold_cpml_batch(b->d_cpml, n, max_np, max_nf, folded,
-                                                (int)(T - folded), rs));
-      ++folds;
+      if (q == T) break;
+      for (int g0 = 0; g0 < n; g0 += fdtd::kCpmlGroup) {
+        const int ng = std::min(n - g0, fdtd::kCpmlGroup);
+        fdtd::CpmlGroup grp;
+        memset(&grp, 0, sizeof(grp));
+        std::copy(hot.begin() + g0, hot.begin() + g0 + ng, grp.h);
+        BCUDA(b, fdtd::launch_cpml_batch_step(grp, ng, b->d_cpml + g0, q, rs));
+      }
     }
     return FDTD_OK;
   };
   b->last_graph = 0;
   if (use_graph) {
-    const std::vector<long long> key = {-1, T, n, max_nx, max_ny, max_nz, max_np, max_nf};
+    std::vector<long long> key = {-1, T, n, max_np, max_nf};
+    const size_t words = hot.size() * sizeof(fdtd::CpmlHot) / sizeof(long long);
+    static_assert(sizeof(fdtd::CpmlHot) % sizeof(long long) == 0, "key words");
+    key.resize(5 + words);
+    memcpy(key.data() + 5, hot.data(), words * sizeof(long long));
     if (!b->gexec || key != b->gkey) {
       if (b->gexec) {
         cudaGraphExecDestroy(b->gexec);
@@ -2021,8 +2063,7 @@ fdtd_status batch_step_cpml(fdtd_batch* b, int64_t T, int32_t use_graph, cudaStr
   if (!b->args_read) BCUDA(b, cudaEventCreateWithFlags(&b->args_read, cudaEventDisableTiming));
   BCUDA(b, cudaEventRecord(b->args_read, st));
   b->args_pending = true;
-  const int per = 65535 / std::max(max_nz, 1);
-  const int launches = (int)(2 * T * ((n + per - 1) / per));
+  const int launches = (int)(2 * T * ngroups);
   for (fdtd_handle* h : b->sims) {
     h->t += T;
     h->last_kernel = 6;  // the per-step CPML kernels

@@ -17,10 +17,6 @@ cudaError_t launch_naive_step(const Grid& g, const FieldPtrs& F, const float* co
                               const Monitors& M, long long t, float dx, cudaStream_t st,
                               int* launches, bool fp64);
 
-// Running-DFT update of every monitor from the current FP32 fields at step t (one launch).
-cudaError_t launch_naive_dft(const Grid& g, const FieldPtrs& F, const Monitors& M, long long t,
-                             cudaStream_t st, int* launches);
-
 // ---------------------------------------------------------------- CPML (cpml.cu)
 // One axis of the CPML profiles: tables over the n positions of the axis, at the E positions
 // (integer n: b, a, 1/kappa of the E updates' differences) and at the H positions (n + 1/2).
@@ -39,32 +35,45 @@ struct CpmlDev {
   float* psi_e[6];
   float* psi_h[6];
 };
-// One step of E then H with CPML layers (FP32 fields, in place), then the monitors.
-cudaError_t launch_cpml_step(const Grid& g, const FieldPtrs& F, const float* const* coef,
-                             const uint16_t* mat, const Material* tab, const Sources& S,
-                             const Monitors& M, const CpmlDev& P, long long t, float dx,
-                             cudaStream_t st, int* launches);
-
-// One grid of a batch of CPML simulations (device-resident array, built by the host per batch
-// step): fields are updated in place; monitor values go to the staging rings (dft_record) and
-// are folded by launch_dft_fold_cpml_batch.  t0 = the grid's step counter at the start of the
-// batch step.
+// One grid with CPML layers (FP32 fields), alone or in a batch (device-resident array, built by
+// the host per batch step): fields are updated in place; monitor values go to the staging rings
+// (dft_record) and are folded by launch_dft_fold / launch_dft_fold_cpml_batch.  t0 = the grid's
+// step counter at the start of the batch step.
 struct CpmlSim {
   Grid g;
-  FieldPtrs F;
-  const float* coef[12];  // pitched per-cell arrays, or all null with a material map
-  const uint16_t* mat;
-  const Material* tab;
+  const float* coef[12];  // pitched per-cell arrays when there is no material map
   Sources S;
   Monitors M;
-  CpmlDev P;
   long long t0;
   float dx;
+  // Material lean_id (when lean) has Ca = Da = 1, one Cb and one Db on all axes.
+  int lean, lean_id;
+  float lean_cb, lean_db;
 };
-// Step t0 + t_offset of every grid: one E launch and one H launch over all grids (blockIdx.z =
-// grid * max_nz + k; cells outside a smaller grid return at once).
-cudaError_t launch_cpml_batch_step(const CpmlSim* sims, int nsims, int max_nx, int max_ny,
-                                   int max_nz, long long t_offset, cudaStream_t st);
+// What every thread of a half step addresses with; passed as kernel parameters, so it does not
+// change between the steps of a batch unless its layers or field sets do.
+struct CpmlHot {
+  Grid g;
+  FieldPtrs F;
+  const uint16_t* mat;  // material map, or null: per-cell coefficients
+  const Material* tab;
+  CpmlDev P;
+  // Cell groups (kCpmlV cells) of a row that touch the lower and the upper x layer, at the E
+  // ([0]) and the H ([1]) positions.
+  int ql[2], qr[2];
+};
+constexpr int kCpmlV = 2;       // consecutive x cells per thread
+constexpr int kCpmlGroup = 32;  // grids per launch of a batch (their CpmlHot are parameters)
+struct CpmlGroup {
+  CpmlHot h[kCpmlGroup];
+};
+// One step of one grid: an E and an H launch.
+cudaError_t launch_cpml_step(const CpmlHot& h, const CpmlSim& s, long long t, cudaStream_t st,
+                             int* launches);
+// Step t0 + t_offset of n grids: an E and an H launch (blockIdx.z = grid).  sims: their
+// arguments in device memory.
+cudaError_t launch_cpml_batch_step(const CpmlGroup& grp, int n, const CpmlSim* sims,
+                                   long long t_offset, cudaStream_t st);
 // The shell companion of the tiled kernel under CPML layers (cpml.cu): one half step (E, or
 // H with h_half) of step t over the cells of `blocks` (int4 {x tile of 32 cells, y tile of 4
 // rows, plane k, unused}) that lie outside the box `inner` ([lo, hi) per axis x, y, z).  Reads
