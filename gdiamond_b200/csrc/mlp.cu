@@ -11,8 +11,9 @@
 //
 // Two GEMM paths compute the same products: tcgen05.mma with a TMEM accumulator (mlp_tc.cu) and
 // the warp-level mma.sync.m16n8k16 kernel below.  The default (AUTO) runs products of >= 1024
-// rows on the first and the 64-row minibatch products of training on the second;
-// fdtd_mlp_set_gemm forces either (the tests cross-check them).  Inference (predict) on the
+// rows on the first and the products of fdtd_mlp_grad on the second, and training epochs in
+// one launch each where the network fits it (mlp_train.cu; the same mma.sync products);
+// fdtd_mlp_set_gemm forces either path (the tests cross-check them).  Inference (predict) on the
 // tcgen05 path runs all layers in one fused kernel when the widths allow (mlp_tc.cu).
 //
 // GEMM: C[M][N] = sum_k opA(m,k) opB(n,k), opX(r,k) = TX ? X[k*ld + r] : X[r*ld + k], so one
@@ -226,19 +227,15 @@ __global__ void col_sum(int M, int N, const float* G, long long g_stride, float*
   db[e * db_stride + c] = s;
 }
 
-// One Adam step on every member's parameters (bias corrections c1 = 1 - b1^t, c2 = 1 - b2^t),
-// refreshing the BF16 copies.
+// One Adam step on every member's parameters, refreshing the BF16 copies.
 __global__ void adam_step(long long n, float* w, const float* g, float* m, float* v,
-                          __nv_bfloat16* wbf, float lr, float b1, float b2, float eps, float c1,
-                          float c2) {
+                          __nv_bfloat16* wbf, AdamStep ad) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+  float wi = w[i], mi = m[i], vi = v[i];
+  adam_update(wi, mi, vi, g[i], ad);
   m[i] = mi;
   v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   w[i] = wi;
   wbf[i] = __float2bfloat16_rn(wi);
 }
@@ -296,6 +293,12 @@ struct fdtd_mlp {
   __nv_bfloat16* gbf[2] = {nullptr, nullptr};  // their BF16 copies
   float* tgt = nullptr;                        // [E][cap][out]
   float* xin = nullptr;                        // FP32 input staging [cap][in]
+  std::vector<__nv_bfloat16*> gl;  // train_epoch: gl[l] [E][cap][dims[l+1]], gradients of layer l
+  // training workspace, kept between calls: row order [E][n], summed losses, bias corrections
+  int* perm = nullptr;
+  float* dloss = nullptr;
+  float2* corr = nullptr;
+  size_t perm_cap = 0, dloss_cap = 0, corr_cap = 0;
   int gemm_kind = FDTD_MLP_GEMM_AUTO;
   mutable cudaError_t launch_err = cudaSuccess;  // first failed tcgen05 launch set-up
   int* d_err = nullptr;  // nonzero when a bounded wait in a GEMM kernel gave up
@@ -326,6 +329,8 @@ void free_workspace(fdtd_mlp* m) {
     m->g[i] = nullptr;
     m->gbf[i] = nullptr;
   }
+  for (auto p : m->gl) cudaFree(p);
+  m->gl.clear();
   cudaFree(m->tgt);
   cudaFree(m->xin);
   m->tgt = nullptr;
@@ -352,6 +357,19 @@ fdtd_status ensure_cap(fdtd_mlp* m, long long rows) {
   MCUDA(m, cudaMalloc(&m->xin, rows * m->dims[0] * sizeof(float)));
   m->cap = rows;
   return FDTD_OK;
+}
+
+// A device array of at least `count` elements, kept in *p (its contents are not).
+template <typename T>
+cudaError_t grow(fdtd_mlp* m, T** p, size_t* cap, size_t count) {
+  if (count <= *cap) return cudaSuccess;
+  cudaError_t e = cudaStreamSynchronize(m->st);
+  if (e != cudaSuccess) return e;
+  cudaFree(*p);
+  *p = nullptr;
+  *cap = 0;
+  if ((e = cudaMalloc(p, count * sizeof(T))) == cudaSuccess) *cap = count;
+  return e;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -473,6 +491,9 @@ void destroy(fdtd_mlp* m) {
   cudaFree(m->adam_v);
   cudaFree(m->wbf);
   cudaFree(m->d_err);
+  cudaFree(m->perm);
+  cudaFree(m->dloss);
+  cudaFree(m->corr);
   cudaFree(m->X);
   cudaFree(m->Y);
   if (m->st) cudaStreamDestroy(m->st);
@@ -695,13 +716,66 @@ fdtd_status fdtd_mlp_train(fdtd_mlp* m, int32_t epochs, int32_t batch, float lr,
   const int mb = (int)std::min<long long>(batch, n);
   fdtd_status s = ensure_cap(m, mb);
   if (s != FDTD_OK) return s;
-  int* perm = nullptr;
-  float* dloss = nullptr;
-  MCUDA(m, cudaMalloc(&perm, (long long)m->E * n * sizeof(int)));
-  MCUDA(m, cudaMalloc(&dloss, (long long)epochs * m->E * sizeof(float)));
+  MCUDA(m, grow(m, &m->perm, &m->perm_cap, (size_t)m->E * n));
+  MCUDA(m, grow(m, &m->dloss, &m->dloss_cap, (size_t)epochs * m->E));
+  int* perm = m->perm;
+  float* dloss = m->dloss;
   MCUDA(m, cudaMemsetAsync(dloss, 0, (long long)epochs * m->E * sizeof(float), m->st));
   std::vector<int> hp((size_t)m->E * n);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  auto corrections = [&] {
+    ++m->adam_t;
+    return make_float2((float)(1.0 - std::pow((double)b1, (double)m->adam_t)),
+                       (float)(1.0 - std::pow((double)b2, (double)m->adam_t)));
+  };
+  // AUTO: the whole epoch in one launch where the network and the batch fit it (mlp_train.cu).
+  const bool fused = m->gemm_kind == FDTD_MLP_GEMM_AUTO &&
+                     fdtd::mlp::train_epoch_supported(m->dims.data(), m->L, mb);
+  fdtd::mlp::TrainArgs ta{};
+  std::vector<float2> hc;
+  if (fused) {
+    if (m->gl.empty()) {
+      m->gl.assign(m->L, nullptr);
+      for (int l = 0; l < m->L; ++l)
+        if (cudaMalloc(&m->gl[l], m->E * m->cap * m->dims[l + 1] * sizeof(__nv_bfloat16)) !=
+            cudaSuccess) {
+          for (auto p : m->gl) cudaFree(p);
+          m->gl.clear();
+          cudaGetLastError();
+          return mfail(m, FDTD_ERR_CUDA, "training workspace allocation failed");
+        }
+    }
+    ta.L = m->L;
+    ta.steps = (int)((n + mb - 1) / mb);
+    ta.batch = mb;
+    for (int l = 0; l <= m->L; ++l) {
+      ta.dims[l] = m->dims[l];
+      ta.act[l] = m->act[l];
+    }
+    for (int l = 0; l < m->L; ++l) {
+      ta.w_off[l] = m->w_off[l];
+      ta.b_off[l] = m->b_off[l];
+      ta.z[l] = m->z[l];
+      ta.gbf[l] = m->gl[l];
+    }
+    ta.P = m->P;
+    ta.n = n;
+    ta.cap = m->cap;
+    ta.perm = perm;
+    ta.X = m->X;
+    ta.Y = m->Y;
+    ta.params = m->params;
+    ta.adam_m = m->adam_m;
+    ta.adam_v = m->adam_v;
+    ta.wbf = m->wbf;
+    ta.lr = lr;
+    ta.b1 = b1;
+    ta.b2 = b2;
+    ta.eps = eps;
+    MCUDA(m, grow(m, &m->corr, &m->corr_cap, (size_t)ta.steps));
+    ta.corr = m->corr;
+    hc.resize(ta.steps);
+  }
   cudaError_t err = cudaSuccess;
   for (int ep = 0; ep < epochs && err == cudaSuccess; ++ep) {
     for (int e = 0; e < m->E; ++e) {  // each member its own shuffle
@@ -712,6 +786,15 @@ fdtd_status fdtd_mlp_train(fdtd_mlp* m, int32_t epochs, int32_t batch, float lr,
     }
     // the previous epoch's gathers are stream-ordered before this copy
     err = cudaMemcpyAsync(perm, hp.data(), hp.size() * sizeof(int), cudaMemcpyHostToDevice, m->st);
+    if (fused) {
+      for (auto& c : hc) c = corrections();
+      if (err == cudaSuccess)
+        err = cudaMemcpyAsync(m->corr, hc.data(), hc.size() * sizeof(float2),
+                              cudaMemcpyHostToDevice, m->st);
+      ta.loss = dloss + (long long)ep * m->E;
+      if (err == cudaSuccess) err = fdtd::mlp::launch_train_epoch(ta, m->E, m->st);
+      continue;
+    }
     for (long long r0 = 0; r0 < n && err == cudaSuccess; r0 += mb) {
       const int M = (int)std::min<long long>(mb, n - r0);
       fdtd::mlp::gather_batch<<<dim3(std::min<unsigned>(fdtd::mlp::nblocks((long long)M * (in + out)), 128u),
@@ -720,22 +803,18 @@ fdtd_status fdtd_mlp_train(fdtd_mlp* m, int32_t epochs, int32_t batch, float lr,
                                                  m->cap * in, m->tgt, m->cap * out);
       forward(m, M, m->cap * in);
       backward(m, M, m->cap * in, m->cap * out, dloss + (long long)ep * m->E);
-      ++m->adam_t;
-      const float c1 = (float)(1.0 - std::pow((double)b1, (double)m->adam_t));
-      const float c2 = (float)(1.0 - std::pow((double)b2, (double)m->adam_t));
+      const float2 c = corrections();
       const long long tot = m->E * m->P;
       fdtd::mlp::adam_step<<<fdtd::mlp::nblocks(tot), 256, 0, m->st>>>(
-          tot, m->params, m->grads, m->adam_m, m->adam_v, m->wbf, lr, b1, b2, eps, c1, c2);
+          tot, m->params, m->grads, m->adam_m, m->adam_v, m->wbf, {lr, b1, b2, eps, c.x, c.y});
       err = cudaGetLastError();
     }
-    // pageable copies are staged before returning, so hp can be refilled next epoch
+    // pageable copies are staged before returning, so hp and hc can be refilled next epoch
   }
   std::vector<float> hl((size_t)epochs * m->E);
   if (err == cudaSuccess)
     err = cudaMemcpyAsync(hl.data(), dloss, hl.size() * sizeof(float), cudaMemcpyDeviceToHost, m->st);
   const cudaError_t e2 = cudaStreamSynchronize(m->st);
-  cudaFree(perm);
-  cudaFree(dloss);
   if (err != cudaSuccess) return mfail(m, FDTD_ERR_CUDA, cudaGetErrorString(err));
   if (e2 != cudaSuccess) return mfail(m, FDTD_ERR_CUDA, cudaGetErrorString(e2));
   if ((s = check_after(m)) != FDTD_OK) return s;

@@ -49,6 +49,18 @@ __device__ __forceinline__ void epilogue_store(const Epilogue& ep, int e, int r,
   if (EPI == kGeluBack) ep.out_bf[e * ep.stride_out + o] = __float2bfloat16_rn(v);
 }
 
+// One Adam step of one parameter (bias corrections c1 = 1 - b1^t, c2 = 1 - b2^t).
+struct AdamStep {
+  float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ void adam_update(float& w, float& m, float& v, float g,
+                                            const AdamStep& a) {
+  // written out, so that every kernel contracts the same products
+  m = __fmaf_rn(1.0f - a.b1, g, __fmul_rn(a.b1, m));
+  v = __fmaf_rn(__fmul_rn(1.0f - a.b2, g), g, __fmul_rn(a.b2, v));
+  w = w - a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+}
+
 // Fused ensemble inference (mlp_tc.cu): every layer of one member for 256 rows per CTA.
 constexpr int kFusedMaxLayers = 8;
 struct FusedArgs {
@@ -67,6 +79,28 @@ struct FusedArgs {
 // dims[0] <= 64; every other width a multiple of 32 up to 256.
 bool mlp_fused_supported(const int* dims, int L);
 cudaError_t launch_mlp_fused(const FusedArgs& a, int members, cudaStream_t st);
+
+// One epoch of minibatch Adam steps for every member in one launch (mlp_train.cu).
+constexpr int kTrainMaxRows = 128, kTrainMaxWidth = 256;
+struct TrainArgs {
+  int L, steps, batch;             // layers, minibatches (the last may be short), rows of one
+  int dims[kFusedMaxLayers + 1];
+  long long w_off[kFusedMaxLayers], b_off[kFusedMaxLayers];
+  long long P, n, cap;             // parameters per member, rows of data, rows of a workspace
+  const int* perm;                 // [members][n]: order of the rows
+  const float *X, *Y;              // [n][dims[0]], [n][dims[L]]
+  float *params, *adam_m, *adam_v;              // [members][P]
+  __nv_bfloat16* wbf;                           // [members][P]
+  __nv_bfloat16* act[kFusedMaxLayers + 1];      // [members][cap][dims[l]], l >= 1
+  float* z[kFusedMaxLayers];                    // [members][cap][dims[l+1]]
+  __nv_bfloat16* gbf[kFusedMaxLayers];          // [members][cap][dims[l+1]]
+  float* loss;                     // [members]: summed squared errors are added
+  const float2* corr;              // [steps]: Adam's bias corrections
+  float lr, b1, b2, eps;
+};
+// Hidden and output widths multiples of 16 up to 256, at most 64 inputs and 128 rows a batch.
+bool train_epoch_supported(const int* dims, int L, int batch);
+cudaError_t launch_train_epoch(const TrainArgs& a, int members, cudaStream_t st);
 
 // tcgen05 GEMM (mlp_tc.cu): C[M][N] (+epilogue) for `members` members on `st`; `err` receives
 // a nonzero word if a bounded wait inside the kernel gave up.  Instantiated for the epilogues

@@ -181,3 +181,26 @@ def test_fused_inference_matches_layer_by_layer(n):
     assert np.all(np.isfinite(p1))
     assert rel(p1, p0) <= 1e-3, rel(p1, p0)
     assert rel(m1, m0) <= 1e-3
+
+
+# Slices of 1 and 2 column groups and idle CTAs (widths 16..256), partial row tiles, a short last
+# batch, one row, the largest batch, odd input widths, one hidden layer and eight layers.
+@pytest.mark.parametrize("dims,members,n,batch", [
+    ((6, 256, 256, 256, 64), 4, 300, 64), ((6, 96, 64), 1, 130, 100), ((7, 16, 16), 2, 65, 64),
+    ((1, 48, 128, 32), 3, 129, 128), ((64, 240, 16), 2, 77, 33), ((5, 32, 16, 48), 1, 5, 1),
+    ((6,) + (32,) * 8, 2, 90, 48), ((6, 256, 144, 64), 5, 200, 128)])
+def test_fused_training_epoch_equals_separate_launches(dims, members, n, batch):
+    """The one-launch epoch runs the products, sums and updates of the launch-per-product path in
+    the same order: parameters after three epochs are equal bit for bit (the summed losses are
+    accumulated with atomics: relative 1e-5)."""
+    x, y = data(n, dims, 3)
+    out = {}
+    for gemm in ("mma_sync", "auto"):
+        net = gd.MLP(dims, members=members, seed=11, gemm=gemm)
+        net.set_data(x, y)
+        loss = np.concatenate([net.train(2, batch=batch, lr=1e-3, seed=4),
+                               net.train(1, batch=batch, lr=3e-4, seed=5)])
+        out[gemm] = (net.get_params(), loss)
+        net.close()
+    assert np.array_equal(out["auto"][0], out["mma_sync"][0])
+    assert np.allclose(out["auto"][1], out["mma_sync"][1], rtol=1e-5)
