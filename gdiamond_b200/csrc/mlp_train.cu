@@ -3,8 +3,11 @@
 // A minibatch step of the ensemble is a chain of small dependent products (64 rows, widths up to
 // 256): as separate launches (gather, 4 forward products, loss, 4 x {weight gradient, column sum,
 // input gradient}, Adam: 20 of them) each one costs a launch, a cold start and a tail for about a
-// microsecond of work.  Here a cluster of 8 CTAs takes one member through every minibatch of the
-// epoch.  The members are independent, so nothing waits outside its cluster.
+// microsecond of work.  Here a cluster of 16 CTAs (8 for more than 4 members) takes one member
+// through every minibatch of the epoch.  The members are independent, so nothing waits outside
+// its cluster.  4 members of 6-256-256-256-64, 4096 rows in batches of 64: 37 us a step instead of
+// 154 (8 CTAs 58, 16 CTAs of 256 threads 45); bound by the latency of the chain (issue slots 27 %
+// busy, fixed-latency and barrier stalls).
 //
 // Split: CTA c owns a slice of 16-column groups of every layer's outputs.  It computes those
 // columns forward (its rows of W_l) and backward (its columns of G_{l-1}), keeps the matching rows
@@ -28,7 +31,9 @@ namespace fdtd {
 namespace mlp {
 namespace {
 
-constexpr int kThreads = 256;  // 8 warps
+constexpr int kThreads = 512;  // 16 warps
+constexpr int kWarps = kThreads / 32;
+constexpr int kUnits = kTrainMaxWidth / 8 / kWarps;  // 8-column units of dW per warp, at most
 constexpr int kRows = kTrainMaxRows, kWidth = kTrainMaxWidth;
 constexpr int LD = kWidth + 8;   // row stride of the row-operand tiles (BF16), conflict-free
 constexpr int LDW = 32 + 8;      // row stride of a column slice of W
@@ -205,7 +210,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
       __syncthreads();
       float loss = 0.0f;
       const int tiles = mt * (count / (8 * NJ));  // 16 rows x 8 NJ columns each
-      for (int t = warp; t < tiles; t += kThreads / 32) {
+      for (int t = warp; t < tiles; t += kWarps) {
         const int m0 = (t % mt) * 16, n0 = (t / mt) * 8 * NJ;
         float2 bv[NJ], yv[NJ][2];  // loaded ahead of the product that hides their latency
 #pragma unroll
@@ -276,7 +281,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
       __syncthreads();
       if (l > 0) {  // G_{l-1} = (G_l W_l) * GELU'(z_{l-1})
         const int tiles = mt * (ccount / (8 * NJ));
-        for (int t = warp; t < tiles; t += kThreads / 32) {
+        for (int t = warp; t < tiles; t += kWarps) {
           const int m0 = (t % mt) * 16, n0 = (t / mt) * 8 * NJ;
           float2 zv[NJ][2];  // loaded ahead of the product that hides their latency
 #pragma unroll
@@ -309,12 +314,12 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
         cluster_arrive();
       }
       // dW_l, rows rfirst.. (at most RT 16-row tiles), this warp's 8-column units
-      const int units = (in16 + 7) / 8, per = (units + 7) / 8;
+      const int units = (in16 + 7) / 8, per = (units + kWarps - 1) / kWarps;
       // The parameters and moments that this thread updates are its own: all of them are loaded
       // now, behind the products and the barrier (one load after another's store would wait for
-      // it, 48 times).
+      // it, for every element).
       const bool even = (in & 1) == 0;
-      float2 pw[RT][4][2], pm[RT][4][2], pv[RT][4][2];
+      float2 pw[RT][kUnits][2], pm[RT][kUnits][2], pv[RT][kUnits][2];
       auto mine = [&](int i, int u, int h, long long* q) {
         const int col = (warp * per + u) * 8 + 2 * tig;
         *q = po + a.w_off[l] + (long long)(rfirst + 16 * i + gid + 8 * h) * in + col;
@@ -323,7 +328,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < kUnits; ++u)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             long long q;
@@ -333,11 +338,11 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
               pv[i][u][h] = *reinterpret_cast<const float2*>(a.adam_v + q);
             }
           }
-      float w[RT][4][4] = {};
+      float w[RT][kUnits][4] = {};
       for (int k = 0; k < M16; k += 16) {
-        uint32_t fb[4][2];
+        uint32_t fb[kUnits][2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < kUnits; ++u)
           if (u < per && warp * per + u < units)
             ldsm2<true>(fb[u], sB + (k + (lane & 15)) * LD + (warp * per + u) * 8);
 #pragma unroll
@@ -348,7 +353,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
             ldsm4<true>(fa, sA + (k + (lane & 7) + ((lane >> 4) & 1) * 8) * LD + rfirst + 16 * i +
                                 ((lane >> 3) & 1) * 8);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < kUnits; ++u)
               if (u < per && warp * per + u < units) mma(w[i][u], fa, fb[u]);
           }
       }
@@ -359,7 +364,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < kUnits; ++u)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             long long q;
