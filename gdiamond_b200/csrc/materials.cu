@@ -6,8 +6,10 @@
 // dielectrics, the graded PML shell), so the solver stores a uint16 id per cell plus a table
 // of distinct tuples.  This file builds that map on the device:
 //   1. insert: hash each cell's 12 words (bitwise) into an open-addressing table of 2^20
-//      64-bit keys; the thread that inserts a key records its cell as the representative;
-//   2. assign: number the occupied slots and copy each representative tuple into the table;
+//      64-bit keys; a key's representative is its first cell (lowest index);
+//   2. assign: number the keys in the order of their representatives and copy each one's tuple
+//      into the table.  Neighbouring cells of a graded layer then have neighbouring table
+//      entries, and a warp's coefficient loads touch a few cache lines instead of one per cell;
 //   3. map: write each cell's id and compare its 12 words with the table entry, so a 64-bit
 //      hash collision is detected (the map is then rejected) instead of silently merged; count
 //      the cells of each id and report the id held by the most cells (the kernels' fast path
@@ -35,6 +37,8 @@ struct Scratch {
   unsigned int flags;  // 1 = probe overflow, 2 = hash collision
   unsigned int mode;   // id held by the most cells (the lowest such id on a tie)
   unsigned int count[kMaxMaterials];  // cells per id
+  uint32_t slot[kMaxMaterials];            // occupied slots, in no order
+  unsigned long long first[kMaxMaterials]; // their representatives
 };
 
 struct Coef12 {
@@ -88,27 +92,45 @@ __global__ void k_insert(Grid g, Coef12 C, Scratch* s, long long n) {
       if (cur == h) { done = true; break; }
       if (cur == kEmpty) {
         const unsigned long long old = atomicCAS(&s->keys[slot], kEmpty, h);
-        if (old == kEmpty) {
-          s->rep[slot] = (unsigned long long)idx;
-          atomicAdd(&s->nuniq, 1u);
-          done = true;
-          break;
-        }
-        if (old == h) { done = true; break; }
+        if (old == kEmpty) atomicAdd(&s->nuniq, 1u);
+        if (old == kEmpty || old == h) { done = true; break; }
       }
       slot = (slot + 1) & (kSlots - 1);
     }
-    if (!done) atomicOr(&s->flags, 1u);
+    if (!done) {
+      atomicOr(&s->flags, 1u);
+      continue;
+    }
+    if ((unsigned long long)idx < *((volatile unsigned long long*)&s->rep[slot]))
+      atomicMin(&s->rep[slot], (unsigned long long)idx);
   }
 }
 
-__global__ void k_assign(Coef12 C, Scratch* s, Material* table) {
+// Lists the occupied slots and their representatives.
+__global__ void k_list(Scratch* s) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= kSlots || s->keys[q] == kEmpty) return;
-  const unsigned int id = atomicAdd(&s->nid, 1u);
-  s->ids[q] = id;
-  if (id >= (unsigned)kMaxMaterials) return;
-  const long long r = (long long)s->rep[q];
+  const unsigned int n = atomicAdd(&s->nid, 1u);
+  if (n >= (unsigned)kMaxMaterials) return;  // rejected on the host
+  s->slot[n] = q;
+  s->first[n] = s->rep[q];
+}
+
+// Entry n of the list gets the id that counts the representatives before its own.
+__global__ void __launch_bounds__(256) k_assign(Coef12 C, Scratch* s, Material* table, int nuniq) {
+  __shared__ unsigned long long tile[256];
+  const int n = blockIdx.x * 256 + threadIdx.x;
+  const unsigned long long r = n < nuniq ? s->first[n] : 0;
+  int id = 0;
+  for (int t0 = 0; t0 < nuniq; t0 += 256) {
+    __syncthreads();
+    if (t0 + (int)threadIdx.x < nuniq) tile[threadIdx.x] = s->first[t0 + threadIdx.x];
+    __syncthreads();
+    const int m = min(256, nuniq - t0);
+    for (int q = 0; q < m; ++q) id += tile[q] < r ? 1 : 0;
+  }
+  if (n >= nuniq) return;
+  s->ids[s->slot[n]] = (uint32_t)id;
   float v[12];
 #pragma unroll
   for (int a = 0; a < 12; ++a) v[a] = C.c[a][r];
@@ -227,7 +249,9 @@ cudaError_t build_material_map(const Grid& g, const float* const* coef12, uint16
   if (e != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   if (hdr[2] != 0 || hdr[0] > (unsigned)kMaxMaterials) return cudaGetLastError();
-  k_assign<<<(kSlots + threads - 1) / threads, threads, 0, st>>>(C, s, table);
+  const int nuniq = (int)hdr[0];
+  k_list<<<(kSlots + threads - 1) / threads, threads, 0, st>>>(s);
+  k_assign<<<(nuniq + 255) / 256, 256, 0, st>>>(C, s, table, nuniq);
   k_map<<<blocks, threads, 0, st>>>(g, C, s, table, mat, n);
   k_mode<<<1, 1024, 0, st>>>(s, (int)hdr[0]);
   unsigned int hdr4[4];
