@@ -358,7 +358,7 @@ std::vector<fdtd::TiledConfig> candidates(const fdtd_handle* h) {
   const bool half = h->esz == 2;
   if (half) {
     fams = {1, 2};
-    rows_l = {8, 16, 24, 32, 48};
+    rows_l = {8, 16, 20, 24, 32, 48};
   }
   if (h->desc.blt > 0) blts = {h->desc.blt};
   if (h->desc.tile_rows > 0) rows_l = {h->desc.tile_rows};
@@ -367,19 +367,31 @@ std::vector<fdtd::TiledConfig> candidates(const fdtd_handle* h) {
   if (h->desc.kernel == FDTD_KERNEL_TILED_W64) fams = {1};
   if (h->desc.kernel == FDTD_KERNEL_TILED_W32P) fams = {2};
   const bool forced_z = h->desc.z_chunks > 0;
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->desc.device);
   for (int fam : fams)
     for (int rows : rows_l)
       for (int b : blts)
-        for (int z : zc)
-          for (int mb : {1, 2, 4}) {
-            if (h->desc.min_blocks > 0 && mb != h->desc.min_blocks) continue;
-            fdtd::TiledConfig c{b, rows, z, fam == 1 ? 64 : 32, mb, h->storage, h->esz};
-            c.pairs32 = fam == 2;
-            if (!config_supported(c)) continue;
+        for (int mb : {1, 2, 4}) {
+          if (h->desc.min_blocks > 0 && mb != h->desc.min_blocks) continue;
+          fdtd::TiledConfig c{b, rows, 1, fam == 1 ? 64 : 32, mb, h->storage, h->esz};
+          c.pairs32 = fam == 2;
+          if (!config_supported(c)) continue;
+          // Grids too small to give every SM a whole column: as many z-chunks as fill one or two
+          // CTAs per SM, too (100^3: 7 planes per chunk instead of 13, 1.2x faster).
+          std::vector<int> zl = zc;
+          const dim3 gd = fam == 0 ? fdtd::tiled_grid(c, h->g) : fdtd::tiled2_grid(c, h->g);
+          for (int k = 1; k <= 2 && !forced_z; ++k) {
+            const int z = (int)((long long)k * nsm / ((long long)gd.x * gd.y));
+            if (z > 1 && std::find(zl.begin(), zl.end(), z) == zl.end()) zl.push_back(z);
+          }
+          for (int z : zl) {
+            c.z_chunks = z;
             // A chunk shorter than its 2*BLT warm-up is only worth it when asked for.
             if (!forced_z && (h->g.nz + z - 1) / z < 2 * b) continue;
             out.push_back(c);
           }
+        }
   return out;
 }
 
@@ -410,19 +422,25 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
   cudaEvent_t e0, e1;
   CUDA_TRY(h, cudaEventCreate(&e0));
   CUDA_TRY(h, cudaEventCreate(&e1));
-  // Time one candidate: one untimed launch, then `reps` timed launches; ms per step.
-  auto time_cfg = [&](const fdtd::TiledConfig& c, int reps, float* per_step) -> fdtd_status {
+  // Time one candidate: one untimed launch, then at least `reps` timed launches and `least` ms of
+  // them; ms per step.
+  auto time_cfg = [&](const fdtd::TiledConfig& c, int reps, float least, float* per_step)
+      -> fdtd_status {
     fdtd_status s = ensure_maps(h, c);
     if (s != FDTD_OK) return s;
     const fdtd::TiledArgs a = make_tiled_args(h, c, 0, false);
     CUDA_TRY(h, launch_any(c, a, h->g, st));
-    CUDA_TRY(h, cudaEventRecord(e0, st));
-    for (int r = 0; r < reps; ++r) CUDA_TRY(h, launch_any(c, a, h->g, st));
-    CUDA_TRY(h, cudaEventRecord(e1, st));
-    CUDA_TRY(h, cudaEventSynchronize(e1));
-    float ms = 0;
-    CUDA_TRY(h, cudaEventElapsedTime(&ms, e0, e1));
-    *per_step = ms / (reps * c.blt);
+    for (int pass = 0; pass < 2; ++pass) {
+      CUDA_TRY(h, cudaEventRecord(e0, st));
+      for (int r = 0; r < reps; ++r) CUDA_TRY(h, launch_any(c, a, h->g, st));
+      CUDA_TRY(h, cudaEventRecord(e1, st));
+      CUDA_TRY(h, cudaEventSynchronize(e1));
+      float ms = 0;
+      CUDA_TRY(h, cudaEventElapsedTime(&ms, e0, e1));
+      *per_step = ms / (reps * c.blt);
+      if (ms >= least) break;
+      reps = std::min(40, (int)(reps * least / std::max(ms, 1e-3f)) + 1);
+    }
     return FDTD_OK;
   };
   // Bring the SM clocks up before anything is compared (an idle GPU starts slow and would
@@ -430,32 +448,58 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
   {
     float warm = 0, spent = 0;
     for (int r = 0; r < 64 && spent < 50.0f; ++r) {
-      fdtd_status s = time_cfg(cands[0], 2, &warm);
+      fdtd_status s = time_cfg(cands[0], 2, 0.0f, &warm);
       if (s != FDTD_OK) return s;
       spent += warm * 2 * cands[0].blt;
     }
   }
+  // First every tile shape at two z-chunk counts (its largest, and 4), then the other counts of
+  // the eight best shapes.
+  auto shape = [](const fdtd::TiledConfig& c) {
+    return std::make_tuple(c.pairs32, c.width, c.rows, c.blt, c.min_blocks);
+  };
+  std::map<std::tuple<bool, int, int, int, int>, int> most;  // largest z-chunk count of a shape
+  for (const auto& c : cands) most[shape(c)] = std::max(most[shape(c)], c.z_chunks);
   std::vector<std::pair<float, size_t>> scored;
-  for (size_t i = 0; i < cands.size(); ++i) {
+  std::vector<bool> timed(cands.size(), false);
+  auto score = [&](size_t i) -> fdtd_status {
     float per_step = 0;
-    fdtd_status s = time_cfg(cands[i], 3, &per_step);
-    if (s != FDTD_OK) return s;
-    scored.emplace_back(per_step, i);
+    timed[i] = true;
+    fdtd_status s = time_cfg(cands[i], 3, 0.2f, &per_step);
+    if (s == FDTD_OK) scored.emplace_back(per_step, i);
+    return s;
+  };
+  for (size_t i = 0; i < cands.size(); ++i)
+    if (cands[i].z_chunks == 4 || cands[i].z_chunks == most[shape(cands[i])]) {
+      fdtd_status s = score(i);
+      if (s != FDTD_OK) return s;
+    }
+  std::sort(scored.begin(), scored.end());
+  std::vector<std::tuple<bool, int, int, int, int>> top;
+  for (const auto& sc : scored) {
+    const auto k = shape(cands[sc.second]);
+    if (top.size() < 8 && std::find(top.begin(), top.end(), k) == top.end()) top.push_back(k);
   }
-  // Re-time the best few with more launches and keep the fastest.
+  for (size_t i = 0; i < cands.size(); ++i)
+    if (!timed[i] && std::find(top.begin(), top.end(), shape(cands[i])) != top.end()) {
+      fdtd_status s = score(i);
+      if (s != FDTD_OK) return s;
+    }
+  // Re-time the best few with more launches, twice in turn, and keep the fastest.
   std::sort(scored.begin(), scored.end());
   float best = 1e30f;
   fdtd::TiledConfig best_c = cands[scored[0].second];
-  for (size_t r = 0; r < std::min<size_t>(4, scored.size()); ++r) {
-    const fdtd::TiledConfig& c = cands[scored[r].second];
-    float per_step = 0;
-    fdtd_status s = time_cfg(c, 8, &per_step);
-    if (s != FDTD_OK) return s;
-    if (per_step < best) {
-      best = per_step;
-      best_c = c;
+  for (int pass = 0; pass < 2; ++pass)
+    for (size_t r = 0; r < std::min<size_t>(5, scored.size()); ++r) {
+      const fdtd::TiledConfig& c = cands[scored[r].second];
+      float per_step = 0;
+      fdtd_status s = time_cfg(c, 8, 0.5f, &per_step);
+      if (s != FDTD_OK) return s;
+      if (per_step < best) {
+        best = per_step;
+        best_c = c;
+      }
     }
-  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   h->cfg = best_c;

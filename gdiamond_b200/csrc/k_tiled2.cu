@@ -9,7 +9,7 @@ namespace {
 bool pairs32_supported(const TiledConfig& c) {
   return (c.esz == 4 || c.esz == 2) && c.width == 32 && c.min_blocks == 1 &&
          ((c.rows == 32 && c.blt >= 1 && c.blt <= 3) ||
-          ((c.rows == 24 || c.rows == 48) && c.blt >= 1 && c.blt <= 2));
+          ((c.rows == 20 || c.rows == 24 || c.rows == 48) && c.blt >= 1 && c.blt <= 2));
 }
 
 }  // namespace

@@ -28,6 +28,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "fdtd_kernels.cuh"
 
 namespace fdtd {
@@ -118,7 +120,6 @@ template <typename S, int B, int TY, int W = 64, typename SH = S>
 struct Tiled2 {
   static constexpr int ESZ_E = (int)sizeof(S);    // stored E value
   static constexpr int ESZ_H = (int)sizeof(SH);   // stored H value
-  static constexpr int ESZ = ESZ_E < ESZ_H ? ESZ_E : ESZ_H;
   static constexpr int LPR = W / 2;            // lanes per tile row
   static constexpr int THREADS = TY * LPR;
   static constexpr int WB = W + kTiled2BoxPad;  // box width of fields and material ids
@@ -131,10 +132,14 @@ struct Tiled2 {
   static constexpr int SX = tiled2_sx_w(W, B);
   static constexpr int SY = tiled_sy(B, TY);
   static constexpr int XBASE = tiled2_xbase(B);
-  static constexpr uint32_t OFF_HPLANES = 3u * PL * ESZ_E;  // H planes follow E in a stage
-  static constexpr uint32_t STAGE_F_BYTES = 3u * PL * (ESZ_E + ESZ_H);
+  // strides of the staged E and H planes in elements: TMA destinations are 128-byte aligned
+  static constexpr int PSE = (PL * ESZ_E + 127) / 128 * 128 / ESZ_E;
+  static constexpr int PSH = (PL * ESZ_H + 127) / 128 * 128 / ESZ_H;
+  static constexpr uint32_t OFF_HPLANES = 3u * PSE * ESZ_E;  // H planes follow E in a stage
+  static constexpr uint32_t STAGE_F_BYTES = 3u * (PSE * ESZ_E + PSH * ESZ_H);
+  static constexpr uint32_t FIELD_BYTES = 3u * PL * (ESZ_E + ESZ_H);  // that the copies deliver
   static constexpr uint32_t STAGE_M_BYTES = MPL_S * 2u;  // TMA destinations stay 128-aligned
-  static constexpr uint32_t TX_BYTES = STAGE_F_BYTES + MPL * 2u;  // bytes the copies deliver
+  static constexpr uint32_t TX_BYTES = FIELD_BYTES + MPL * 2u;  // with the material ids
   static constexpr size_t OFF_M = (size_t)NS * STAGE_F_BYTES;
   static constexpr size_t OFF_H = OFF_M + (size_t)NS * STAGE_M_BYTES;
   static constexpr size_t OFF_E = OFF_H + 2u * 2u * PLX * 4u;
@@ -144,9 +149,40 @@ struct Tiled2 {
   static_assert(SX % 2 == 0 && XBASE % 2 == 0 && XBASE + B <= 0, "even tile starts");
   static_assert(SY >= 1, "tile too short for this BLT");
   static_assert((W == 64 || W == 32) && THREADS % 32 == 0, "warp rows of 64 or 32 cells");
-  static_assert(STAGE_M_BYTES % 128 == 0 && (PL * ESZ) % 128 == 0, "stage alignment");
+  static_assert(STAGE_M_BYTES % 128 == 0, "stage alignment");
   static_assert(STAGE_F_BYTES % 128 == 0, "stage alignment");
 };
+
+// Sources of components c0 .. c0+2 at the x-pair (x0, y, k) and step t: curl -= (sum of the
+// covering waveforms) * dx per component and cell, as source_value sums them, in one loop over the
+// sources (six copies of that loop per half level made the mixed march's code a third longer).
+__device__ __forceinline__ void add_sources(const Sources& S, int c0, int x0, int y, int k,
+                                            long long t, float dx, float2& cx, float2& cy,
+                                            float2& cz) {
+  float2 acc[3] = {};
+  unsigned any = 0;  // bit 2 c + cell
+  for (int n = 0; n < S.n; ++n) {
+    const SourceDev& s = S.s[n];
+    const int c = s.comp - c0;
+    if (c < 0 || c > 2 || s.k != k || (s.kind == 0 && (s.j != y || (s.i != x0 && s.i != x0 + 1))))
+      continue;
+    const float w = t < S.tw ? S.wave[n * S.tw + t] : 0.0f;
+    const bool h0 = s.kind != 0 || s.i == x0, h1 = s.kind != 0 || s.i == x0 + 1;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      if (q != c) continue;
+      if (h0) acc[q].x = add(acc[q].x, w);
+      if (h1) acc[q].y = add(acc[q].y, w);
+    }
+    any |= ((h0 ? 1u : 0u) | (h1 ? 2u : 0u)) << (2 * c);
+  }
+  if (any & 1u) cx.x = sub(cx.x, mul(acc[0].x, dx));
+  if (any & 2u) cx.y = sub(cx.y, mul(acc[0].y, dx));
+  if (any & 4u) cy.x = sub(cy.x, mul(acc[1].x, dx));
+  if (any & 8u) cy.y = sub(cy.y, mul(acc[1].y, dx));
+  if (any & 16u) cz.x = sub(cz.x, mul(acc[2].x, dx));
+  if (any & 32u) cz.y = sub(cz.y, mul(acc[2].y, dx));
+}
 
 __device__ __forceinline__ float2 ldf2(const float* p) {
   return *reinterpret_cast<const float2*>(p);
@@ -264,15 +300,15 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
     const uint32_t u = gbase + (uint32_t)it_;
     const int stage = (int)(u % K::NS);
     uint64_t* bar = &bars[stage];
-    mbar_arrive_expect_tx(bar, LO ? K::STAGE_F_BYTES : K::TX_BYTES);
+    mbar_arrive_expect_tx(bar, LO ? K::FIELD_BYTES : K::TX_BYTES);
     unsigned char* d = st_f + stage * K::STAGE_F_BYTES;
     S* de = reinterpret_cast<S*>(d);
     SH* dh = reinterpret_cast<SH*>(d + K::OFF_HPLANES);
     const int pz = ps + it_;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      tma_load_3d(de + c * K::PL, &a.tm_src[c], bar, X8, Y, pz);
-      tma_load_3d(dh + c * K::PL, &a.tm_src[3 + c], bar, X8, Y, pz);
+      tma_load_3d(de + c * K::PSE, &a.tm_src[c], bar, X8, Y, pz);
+      tma_load_3d(dh + c * K::PSH, &a.tm_src[3 + c], bar, X8, Y, pz);
     }
     if (!LO) tma_load_3d(st_m + stage * K::MPL_S, &a.tm_mat, bar, X8, Y, pz);
   };
@@ -307,17 +343,17 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
   uint32_t seen_e = 0, seen_h = 0;  // 16-bit storage: running max |stored value| (see Store)
   int it = 0;
   bool abort = false;
-  for (; it < niter; ++it) {
-    const int p = ps + it;
-    const uint32_t u = gbase + (uint32_t)it;
-    const int stage = (int)(u % K::NS);
-    if (!mbar_wait_bounded(&bars[stage], (u / K::NS) & 1u, wait_limit)) {
-      *sm.abort = 1;
-      atomicOr(a.err, kErrTimeout);
-    }
-    if (B == 1) __syncthreads();  // orders last iteration's ebuf writes before this read
-    const bool mon_iter = p >= mon_lo && p <= mon_hi;
-    const bool src_iter = smask != 0 && p >= src_lo && p <= src_hi;
+  // One z-iteration on the staged plane p.  SP (special): some level may touch a source, a
+  // monitor or a z face.  The other iterations, nearly all, run a copy of the code without any of
+  // those tests (256^3 vacuum, BLT 3: 155 Gcell-updates/s, 143 with one copy).  Longer unrolling
+  // is slower although it removes the moves between registers (NP = BLT + 1 iterations with the
+  // planes' registers renamed: 362 instead of 410 instructions per iteration, but the loop no
+  // longer fits the instruction cache and runs at 124).  Returns false when a bounded wait has
+  // expired.
+  auto iteration = [&](auto special, int p, int stage) -> bool {
+    constexpr bool SP = decltype(special)::value;
+    const bool mon_iter = SP && p >= mon_lo && p <= mon_hi;
+    const bool src_iter = SP && smask != 0 && p >= src_lo && p <= src_hi;
 
     const S* E0 = reinterpret_cast<const S*>(st_f + stage * K::STAGE_F_BYTES);
     const SH* H0 = reinterpret_cast<const SH*>(st_f + stage * K::STAGE_F_BYTES + K::OFF_HPLANES);
@@ -327,15 +363,16 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
       for (int s = B; s >= 1; --s) mq[s] = mq[s - 1];
       mq[0] = *reinterpret_cast<const uint32_t*>(st_m + stage * K::MPL_S + om);
       uh = (uh << 1) | (__all_sync(kFull, mq[0] == lean_ids) ? 1u : 0u);
-      lean = lean_on && (uh & kPlanes) == kPlanes && p >= B + 1 && p <= g.nz - 2 && !src_iter;
+      lean = lean_on && (uh & kPlanes) == kPlanes &&
+             (!SP || (p >= B + 1 && p <= g.nz - 2 && !src_iter));
     }
     float2 Hc[3], Eo[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      Hc[c] = StH::ld2(H0 + c * K::PL + os, sc[3 + c]);
-      Eo[c] = St::ld2(E0 + c * K::PL + os, sc[c]);
+      Hc[c] = StH::ld2(H0 + c * K::PSH + os, sc[3 + c]);
+      Eo[c] = St::ld2(E0 + c * K::PSE + os, sc[c]);
     }
-    float2 hz_ym = StH::ld2(H0 + 2 * K::PL + osym, sc[5]);
+    float2 hz_ym = StH::ld2(H0 + 2 * K::PSH + osym, sc[5]);
     float2 hx_ym = StH::ld2(H0 + osym, sc[3]);
     float2 EnPrev[3] = {};
     float2 EnB[3] = {}, HnB[3] = {};
@@ -364,7 +401,7 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
         En[0] = add2(Eo[0], scale2(a.lean_cb, ex_c));
         En[1] = add2(Eo[1], scale2(a.lean_cb, ey_c));
         En[2] = add2(Eo[2], scale2(a.lean_cb, ez_c));
-        const bool ke = !LO || (e >= 1 && e <= g.nz - 2);  // mixed tiles: lean only off z faces
+        const bool ke = !(SP && LO) || (e >= 1 && e <= g.nz - 2);  // mixed tiles: lean only off z faces
         if (wface || !ke) {  // face and outside cells keep their value
           const bool u0 = int0 && ke, u1 = int1 && ke;
 #pragma unroll
@@ -380,7 +417,7 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
         Hn[0] = add2(Hp[s - 1][0], scale2(a.lean_db, hx_c));
         Hn[1] = add2(Hp[s - 1][1], scale2(a.lean_db, hy_c));
         Hn[2] = add2(Hp[s - 1][2], scale2(a.lean_db, hz_c));
-        const bool kh = !LO || (e - 1 >= 1 && e - 1 <= g.nz - 2);
+        const bool kh = !(SP && LO) || (e - 1 >= 1 && e - 1 <= g.nz - 2);
         if (wface || !kh) {
           const bool u0 = int0 && kh, u1 = int1 && kh;
 #pragma unroll
@@ -401,15 +438,9 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
         En[0] = Eo[0];
         En[1] = Eo[1];
         En[2] = Eo[2];
-        if (e >= 1 && e <= g.nz - 2) {
+        if (!SP || (e >= 1 && e <= g.nz - 2)) {
           if (src_iter) {
-            float v;
-            if (source_value(a.S, 0, x0, y, e, t, &v)) cxp.x = sub(cxp.x, mul(v, dx));
-            if (source_value(a.S, 1, x0, y, e, t, &v)) cyp.x = sub(cyp.x, mul(v, dx));
-            if (source_value(a.S, 2, x0, y, e, t, &v)) czp.x = sub(czp.x, mul(v, dx));
-            if (source_value(a.S, 0, x1, y, e, t, &v)) cxp.y = sub(cxp.y, mul(v, dx));
-            if (source_value(a.S, 1, x1, y, e, t, &v)) cyp.y = sub(cyp.y, mul(v, dx));
-            if (source_value(a.S, 2, x1, y, e, t, &v)) czp.y = sub(czp.y, mul(v, dx));
+            add_sources(a.S, 0, x0, y, e, t, dx, cxp, cyp, czp);
           }
           const Material* m0 = a.table + (mq[s - 1] & 0xFFFFu);
           const Material* m1 = a.table + (mq[s - 1] >> 16);
@@ -438,15 +469,9 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
         Hn[0] = Hp[s - 1][0];
         Hn[1] = Hp[s - 1][1];
         Hn[2] = Hp[s - 1][2];
-        if (e - 1 >= 1 && e - 1 <= g.nz - 2) {
+        if (!SP || (e - 1 >= 1 && e - 1 <= g.nz - 2)) {
           if (src_iter) {
-            float v;
-            if (source_value(a.S, 3, x0, y, e - 1, t, &v)) cxp.x = sub(cxp.x, mul(v, dx));
-            if (source_value(a.S, 4, x0, y, e - 1, t, &v)) cyp.x = sub(cyp.x, mul(v, dx));
-            if (source_value(a.S, 5, x0, y, e - 1, t, &v)) czp.x = sub(czp.x, mul(v, dx));
-            if (source_value(a.S, 3, x1, y, e - 1, t, &v)) cxp.y = sub(cxp.y, mul(v, dx));
-            if (source_value(a.S, 4, x1, y, e - 1, t, &v)) cyp.y = sub(cyp.y, mul(v, dx));
-            if (source_value(a.S, 5, x1, y, e - 1, t, &v)) czp.y = sub(czp.y, mul(v, dx));
+            add_sources(a.S, 3, x0, y, e - 1, t, dx, cxp, cyp, czp);
           }
           const Material* m0 = a.table + (mq[s] & 0xFFFFu);
           const Material* m1 = a.table + (mq[s] >> 16);
@@ -522,9 +547,8 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
           HnB[c] = Hn[c];
         }
       }
-      if (abort) break;
+      if (abort) return false;
     }
-    if (abort) break;
 #pragma unroll
     for (int c = 0; c < 3; ++c) Ep[B][c] = EnPrev[c];
 
@@ -555,6 +579,27 @@ __device__ __forceinline__ bool march(const TiledArgs& a, int bx, int by, int bz
         for (int c = 0; c < 3; ++c)
           StH::st1(dsth[c] + idx_h + q, q ? HnB[c].y : HnB[c].x, inv[3 + c], seen_h);
       }
+    }
+    __syncwarp();  // lanes that stored differently: without it they stay apart for a while
+    return true;
+  };
+  uint32_t stage = gbase % K::NS, phase = (gbase / K::NS) & 1u;  // of iteration `it`
+  for (; it < niter; ++it) {
+    const int p = ps + it;
+    if (!mbar_wait_bounded(&bars[stage], phase, wait_limit)) {
+      *sm.abort = 1;
+      atomicOr(a.err, kErrTimeout);
+    }
+    if (B == 1) __syncthreads();  // orders last iteration's ebuf writes before this read
+    // CTA-uniform: levels 1..B work on planes p-B..p
+    const bool sp = p < B + 1 || p > g.nz - 2 || (p >= src_lo && p <= src_hi) ||
+                    (p >= mon_lo && p <= mon_hi);
+    if (!(sp ? iteration(std::true_type{}, p, (int)stage)
+             : iteration(std::false_type{}, p, (int)stage)))
+      break;
+    if (++stage == K::NS) {
+      stage = 0;
+      phase ^= 1u;
     }
   }
 
@@ -642,11 +687,11 @@ __global__ void __launch_bounds__(TY * W / 2, MINB)
     (void)march<S, B, TY, W, SH, false>(a, bx, by, bz, sm, gbase, 0);
 }
 
-// CTAs per SM the compiler must fit: two for the 24-row tiles of 32-cell rows (384 threads, the
-// register budget of the 48-row instance), one otherwise.
+// CTAs per SM the compiler must fit: two for the 20- and 24-row tiles of 32-cell rows (320 and
+// 384 threads), one otherwise.
 template <int TY, int W>
 constexpr int batch_min_blocks() {
-  return (W == 32 && TY == 24) ? 2 : 1;
+  return (W == 32 && (TY == 20 || TY == 24)) ? 2 : 1;
 }
 
 // A batch of independent grids: persistent CTAs pull (grid, tile) work items from a queue.
@@ -694,11 +739,20 @@ cudaError_t launch_batch_one(const BatchArgs& b, int ctas, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// 32-wide rows (two per warp): 24 rows (12 warps, BLT 1-2, registers capped for two CTAs per
-// SM), 32 rows (16 warps, BLT 1-3) or 48 rows (24 warps, BLT 1-2).
+// 32-wide rows (two per warp): 20 and 24 rows (10 and 12 warps, BLT 1-2, registers capped for two
+// CTAs per SM), 32 rows (16 warps, BLT 1-3) or 48 rows (24 warps, BLT 1-2).  Two CTAs wait at
+// barriers of their own, so one computes while the other waits; at 20 rows the 96 registers left
+// to a thread hold BLT 2 without spills, at 24 rows the 80 do not (256^3, 80 spheres, BLT 2: 20
+// rows 124 Gcell-updates/s, 24 rows 106, 32 rows 114).
 template <typename S, typename SH = S>
 cudaError_t launch_pairs32(int blt, int rows, const TiledArgs& a, dim3 grid, cudaStream_t st) {
-  if (rows == 24) {
+  if (rows == 20) {
+    switch (blt) {
+      case 1: return launch_one2<S, 1, 20, 2, 32, SH>(a, grid, st);
+      case 2: return launch_one2<S, 2, 20, 2, 32, SH>(a, grid, st);
+      default: break;
+    }
+  } else if (rows == 24) {
     switch (blt) {
       case 1: return launch_one2<S, 1, 24, 2, 32, SH>(a, grid, st);
       case 2: return launch_one2<S, 2, 24, 2, 32, SH>(a, grid, st);
@@ -724,7 +778,13 @@ cudaError_t launch_pairs32(int blt, int rows, const TiledArgs& a, dim3 grid, cud
 template <typename S, typename SH = S>
 cudaError_t launch_batch_pairs32(int blt, int rows, const BatchArgs& b, int ctas,
                                  cudaStream_t st) {
-  if (rows == 24) {
+  if (rows == 20) {
+    switch (blt) {
+      case 1: return launch_batch_one<S, 1, 20, 32, SH>(b, ctas, st);
+      case 2: return launch_batch_one<S, 2, 20, 32, SH>(b, ctas, st);
+      default: break;
+    }
+  } else if (rows == 24) {
     switch (blt) {
       case 1: return launch_batch_one<S, 1, 24, 32, SH>(b, ctas, st);
       case 2: return launch_batch_one<S, 2, 24, 32, SH>(b, ctas, st);
@@ -852,7 +912,12 @@ size_t batch_query(const TiledConfig& c) {
 #define GD_Q(B, TY, W) (OCC ? (size_t)occupancy_of<S, B, TY, W, SH>() : smem_of<S, B, TY, W, SH>())
   constexpr bool f32 = sizeof(S) == 4 && sizeof(SH) == 4;
   if (c.pairs32) {
-    if (c.rows == 24) {
+    if (c.rows == 20) {
+      switch (c.blt) {
+        case 1: return GD_Q(1, 20, 32);
+        case 2: return GD_Q(2, 20, 32);
+      }
+    } else if (c.rows == 24) {
       switch (c.blt) {
         case 1: return GD_Q(1, 24, 32);
         case 2: return GD_Q(2, 24, 32);

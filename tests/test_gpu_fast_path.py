@@ -130,3 +130,39 @@ def test_fast_path_in_batches():
     for n, (_, _, _, F_ref) in enumerate(refs):
         assert_fields_match(results[True][n], F_ref, f"batch fast {n}")
         assert_fields_match(results[False][n], F_ref, f"batch general {n}")
+
+
+# The 20-row tiles of the x-pair kernel (two CTAs per SM).
+@pytest.mark.parametrize("medium", ["vacuum", "spheres"])
+@pytest.mark.parametrize("blt", [1, 2])
+def test_20_row_tiles_equal_general_path_and_oracle(blt, medium):
+    test_fast_path_equals_general_path_and_oracle("tiled_w32p", blt, 20, medium)
+
+
+@pytest.mark.parametrize("rows,blt", [(20, 2), (32, 3), (20, 1)])
+def test_stacked_sources_match_oracle(rows, blt):
+    """Eight sources: three of one component on one cell, both cells of an x-pair, planes over
+    points, E and H components, one on a pair that straddles a tile edge, one on a face (ignored)
+    -- the sums per cell are formed in the order of the list."""
+    shape, T = (70, 41, 23), 11
+    nx, ny, nz = shape
+    coefs = W.reference_coefficients(shape, eps_re=W.spheres_eps(shape, n_spheres=4, r_range=(3, 6),
+                                                                 seed=2), t_pml=6)
+    w = [W.gaussian_wave(T, delay=3.0 + q, width=2.0, period=5.0) for q in range(8)]
+    src = [dict(component="Jz", wave=w[0], i=30, j=20, k=11),
+           dict(component="Jz", wave=w[1], i=30, j=20, k=11),
+           dict(component="Jz", wave=w[2], i=31, j=20, k=11),
+           dict(component="Jz", wave=w[3] * np.float32(0.1), k=11, kind=gd.SRC_PLANE_Z),
+           dict(component="Jx", wave=w[4], i=28, j=16, k=10),
+           dict(component="Mx", wave=w[5], i=31, j=20, k=11),
+           dict(component="My", wave=w[6][:7], k=5, kind=gd.SRC_PLANE_Z),
+           dict(component="Jy", wave=w[7], i=0, j=20, k=11)]
+    F_ref = oracle.run(shape, coefs, T, sources=[osrc(s) for s in src])
+    for kw in (dict(kernel="tiled_w32p", blt=blt, tile_rows=rows, z_chunks=2), dict(kernel="naive")):
+        sim = gd.Simulation(*shape, **kw)
+        sim.set_coefficients(coefs)
+        sim.set_sources(src)
+        sim.step(T)
+        sim.sync()
+        assert_fields_match(sim.fields(), F_ref, str(kw))
+        sim.close()

@@ -345,3 +345,9 @@ def test_16bit_overflow_is_reported_not_silent(storage):
     for c, f in enumerate(sim.fields()):
         assert bits_equal(f, F_ref[c]), (storage, c)
     sim.close()
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16e"])
+@pytest.mark.parametrize("blt", [1, 2])
+def test_16bit_20_row_tiles_match_rounded_oracle(storage, blt):
+    test_16bit_pairs32_matches_rounded_oracle(storage, blt, 20)

@@ -104,3 +104,9 @@ def test_output_windows_tile_the_grid():
                         cover[x] += 1
             assert (cover == 1).all()
             assert xbase + blt + ntx * sx >= nx and nty * sy >= ny and nzc * zlen >= nz
+
+
+@pytest.mark.parametrize("blt", [1, 2])
+@pytest.mark.parametrize("zc", [1, 3])
+def test_schedule_of_20_row_tiles(blt, zc):
+    test_schedule_point_sources(blt, 20, zc, 32, True)
