@@ -71,6 +71,36 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
   return fn;
 }
 
+// Whether [p, p + bytes) lies in one allocation of `device`'s own memory: a kernel on that device
+// may then access it.  (A caller's buffer may also be pinned or managed host memory, another
+// device's, or too small; the runtime's copy deals with those or reports them.)
+bool own_device_memory(const void* p, size_t bytes, int device) {
+  static PFN_cuPointerGetAttributes_v7000 fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* q = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &q, cudaEnableDefault, &r) ==
+            cudaSuccess &&
+        r == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_cuPointerGetAttributes_v7000>(q);
+  });
+  if (!fn) return false;
+  unsigned int type = 0, managed = 1;
+  int ordinal = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                 CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* out[5] = {&type, &managed, &ordinal, &start, &size};
+  const CUdeviceptr a = reinterpret_cast<CUdeviceptr>(p);
+  if (fn(5, what, out, a) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == device && start && a >= start &&
+         a + bytes <= start + size;
+}
+
 // Process-wide autotuning cache keyed by grid shape.
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, long long>, fdtd::TiledConfig> g_tune_cache;
@@ -200,6 +230,18 @@ struct DeviceGuard {
 
 cudaStream_t pick_stream(fdtd_handle* h, void* s) {
   return s ? static_cast<cudaStream_t>(s) : h->stream;
+}
+
+// `rows` rows of `row` bytes between a field array of h (row stride `pitch`) and a caller's packed
+// device buffer.
+cudaError_t copy_device_rows(const fdtd_handle* h, void* dst, size_t dst_stride, const void* src,
+                             size_t src_stride, size_t row, size_t rows, const void* caller,
+                             cudaStream_t st) {
+  if (own_device_memory(caller, row * rows, h->desc.device))
+    return fdtd::copy_rows(src, (long long)src_stride, dst, (long long)dst_stride, (long long)row,
+                           (long long)rows, st);
+  return cudaMemcpy2DAsync(dst, dst_stride, src, src_stride, row, rows, cudaMemcpyDeviceToDevice,
+                           st);
 }
 
 fdtd_status encode_map(fdtd_handle* h, CUtensorMap* m, void* base, CUtensorMapDataType dt,
@@ -1255,18 +1297,29 @@ fdtd_status fdtd_flux_monitor_ids(const fdtd_handle* h, int32_t flux_id, int32_t
 fdtd_status fdtd_reset(fdtd_handle* h) {
   if (!h) return FDTD_ERR_INVALID_ARG;
   DeviceGuard dg(h->desc.device);
-  for (int s = 0; s < h->nsets; ++s)
-    for (int c = 0; c < 6; ++c)
-      CUDA_TRY(h, cudaMemsetAsync(h->F[s][c], 0, h->cells * comp_esz(h, c), h->stream));
-  for (int m = 0; m < h->nmon; ++m) {
+  // One launch for everything.  The second field set needs no clearing: a step writes every cell
+  // of the set it ends in before reading it, and the pad columns of both sets are never changed.
+  fdtd::ClearList L;
+  L.n = 0;
+  auto clear = [&](void* p, size_t bytes) -> fdtd_status {
+    L.p[L.n] = p;
+    L.bytes[L.n] = bytes;
+    if (++L.n == fdtd::kClearMax) {
+      CUDA_TRY(h, fdtd::clear_ranges(L, h->stream));
+      L.n = 0;
+    }
+    return FDTD_OK;
+  };
+  fdtd_status s = FDTD_OK;
+  for (int c = 0; c < 6 && s == FDTD_OK; ++c) s = clear(h->F[0][c], h->cells * comp_esz(h, c));
+  for (int m = 0; m < h->nmon && s == FDTD_OK; ++m) {
     const size_t bytes = (size_t)h->mon[m].nf * h->g.nx * h->g.ny * sizeof(double);
-    CUDA_TRY(h, cudaMemsetAsync(h->mon[m].re, 0, bytes, h->stream));
-    CUDA_TRY(h, cudaMemsetAsync(h->mon[m].im, 0, bytes, h->stream));
+    if ((s = clear(h->mon[m].re, bytes)) == FDTD_OK) s = clear(h->mon[m].im, bytes);
   }
-  if (h->cpml_on) {
-    for (int q = 0; q < 12; ++q)
-      CUDA_TRY(h, cudaMemsetAsync(h->cpml_psi[q], 0, cpml_psi_bytes(h, q), h->stream));
-  }
+  if (h->cpml_on)
+    for (int q = 0; q < 12 && s == FDTD_OK; ++q) s = clear(h->cpml_psi[q], cpml_psi_bytes(h, q));
+  if (s != FDTD_OK) return s;
+  CUDA_TRY(h, fdtd::clear_ranges(L, h->stream));
   h->t = 0;
   h->cur = 0;
   return FDTD_OK;
@@ -1493,12 +1546,19 @@ fdtd_status fdtd_get_field_device(fdtd_handle* h, int32_t component, float* dev_
   if (!h || !dev_out || component < 0 || component > 5) return FDTD_ERR_INVALID_ARG;
   DeviceGuard dg(h->desc.device);
   cudaStream_t st = pick_stream(h, stream);
+  const int cs = comp_storage(h, component);
+  const size_t bytes = (size_t)h->g.nx * h->g.ny * h->g.nz * sizeof(float);
+  if (cs != FDTD_STORE_F32 && reinterpret_cast<uintptr_t>(dev_out) % alignof(float) == 0 &&
+      own_device_memory(dev_out, bytes, h->desc.device)) {  // straight into the caller's buffer
+    CUDA_TRY(h, fdtd::widen_field_packed(h->g, h->F[h->cur][component], cs, h->scale[component],
+                                         dev_out, st));
+    return FDTD_OK;
+  }
   const float* src = nullptr;
   fdtd_status s = f32_view(h, component, st, &src);
   if (s != FDTD_OK) return s;
-  CUDA_TRY(h, cudaMemcpy2DAsync(dev_out, (size_t)h->g.nx * 4, src, (size_t)h->g.pitch * 4,
-                                (size_t)h->g.nx * 4, (size_t)h->g.ny * h->g.nz,
-                                cudaMemcpyDeviceToDevice, st));
+  CUDA_TRY(h, copy_device_rows(h, dev_out, (size_t)h->g.nx * 4, src, (size_t)h->g.pitch * 4,
+                               (size_t)h->g.nx * 4, (size_t)h->g.ny * h->g.nz, dev_out, st));
   return FDTD_OK;
 }
 
@@ -1563,9 +1623,9 @@ fdtd_status plane_copy(fdtd_handle* h, int32_t comp, int64_t k0, int64_t nk, voi
   const size_t row = (size_t)h->g.nx * esz, pitch = (size_t)h->g.pitch * esz;
   const size_t rows = (size_t)h->g.ny * (size_t)nk;
   if (to_handle)
-    CUDA_TRY(h, cudaMemcpy2DAsync(field, pitch, packed, row, row, rows, cudaMemcpyDeviceToDevice, st));
+    CUDA_TRY(h, copy_device_rows(h, field, pitch, packed, row, row, rows, packed, st));
   else
-    CUDA_TRY(h, cudaMemcpy2DAsync(packed, row, field, pitch, row, rows, cudaMemcpyDeviceToDevice, st));
+    CUDA_TRY(h, copy_device_rows(h, packed, row, field, pitch, row, rows, packed, st));
   return FDTD_OK;
 }
 

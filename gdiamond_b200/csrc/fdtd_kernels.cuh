@@ -91,10 +91,26 @@ cudaError_t launch_cpml_region(bool h_half, const Grid& g, const FieldPtrs& Fi,
 cudaError_t launch_dft_fold_cpml_batch(const CpmlSim* sims, int nsims, long long max_np,
                                        int max_nf, long long t_offset, int n, cudaStream_t st);
 
+// ---------------------------------------------------------------- copies and clears (convert.cu)
+// `rows` rows of `row` bytes from src to dst (row strides in bytes), both on the current device.
+cudaError_t copy_rows(const void* src, long long src_stride, void* dst, long long dst_stride,
+                      long long row, long long rows, cudaStream_t st);
+constexpr int kClearMax = 48;
+struct ClearList {
+  int n;
+  void* p[kClearMax];  // 16-byte aligned
+  unsigned long long bytes[kClearMax];
+};
+// Zeroes every range, one launch.
+cudaError_t clear_ranges(const ClearList& L, cudaStream_t st);
+
 // ---------------------------------------------------------------- storage conversion
 // Pitched field array of `storage` (0 FP32, 1 FP16, 2 BF16, 3 FP64) <-> pitched FP32 / FP64.
 cudaError_t convert_field_to_f32(const Grid& g, const void* src, int storage, float scale,
                                  float* dst, cudaStream_t st);
+// The same into a packed FP32 array [nz][ny][nx] (storage 1, 2 or 3).
+cudaError_t widen_field_packed(const Grid& g, const void* src, int storage, float scale,
+                               float* dst, cudaStream_t st);
 cudaError_t convert_field_from_f32(const Grid& g, const float* src, int storage, float inv_scale,
                                    void* dst, cudaStream_t st);
 cudaError_t convert_field_to_f64(const Grid& g, const void* src, int storage, float scale,
