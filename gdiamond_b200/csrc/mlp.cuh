@@ -61,7 +61,7 @@ __device__ __forceinline__ void adam_update(float& w, float& m, float& v, float 
   w = w - a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
 }
 
-// Fused ensemble inference (mlp_tc.cu): every layer of one member for 256 rows per CTA.
+// Fused ensemble inference (mlp_tc.cu): every layer of one member for 128 rows per CTA.
 constexpr int kFusedMaxLayers = 8;
 struct FusedArgs {
   const float* x;                  // [n][dims[0]] FP32 inputs

@@ -18,6 +18,7 @@
 // Every mbarrier wait is bounded; on expiry the kernel records an error word, stops issuing
 // (decided block-wide with __syncthreads_or), waits (bounded) for what it issued, skips the
 // epilogue, frees its TMEM and returns.
+#include <algorithm>
 #include <atomic>
 
 #include "fdtd_common.cuh"
@@ -305,20 +306,27 @@ cudaError_t launch_bn(int M, int N, int K, const Operand& A, const Operand& B, c
 }
 
 // ------------------------------------------------------------------- fused ensemble inference
-// One CTA of 256 threads takes 256 rows (two 128-row tiles) of one member through every layer:
-// the BF16 activations stay in shared memory as the next layer's A operand (one 128 x 256 K-major
-// core-matrix tile per row tile, 8-row groups 4096 B apart), the weights stream through two
-// 64-wide K stages (N x 64 core matrices) and each staged chunk feeds both row tiles, the FP32
-// accumulators (up to 2 x 256 columns) stay in TMEM, and only the last layer's output is written
-// to global memory.  Warps 0-3 run the epilogue of tile 0, warps 4-7 that of tile 1.
+// One CTA of 256 threads takes 128 rows of one member through every layer: the BF16 activations
+// stay in shared memory as the next layer's A operand (a 128 x 256 K-major core-matrix tile,
+// 8-row groups 4096 B apart), the weights pass through a 64-wide K stage (N x 64 core matrices),
+// the FP32 accumulator (up to 256 columns) stays in TMEM, and only the last layer's output is
+// written to global memory.  Warp w runs the epilogue of rows 32 (w % 4) .. +31, every second
+// 32-column group.
+//
+// Bound: issue slots of the epilogue (bias, erf, rounding: about 40 instructions per hidden value
+// against 2 * 256 multiply-adds of the tensor core), so what counts is that some warps are in an
+// epilogue while others stage weights or wait for products: two CTAs per SM, each with half of
+// the TMEM and 97 KB, instead of one CTA with two row tiles.  The biases are read from shared
+// memory, four at a time.
 
 constexpr int FACT_K = 256;  // widest layer input held in the activation tile
-constexpr int FROWS = 128;                             // rows of one tile (the MMA's M)
-constexpr int FTILES = 2;                              // row tiles per CTA
+constexpr int FROWS = 128;                             // rows of a CTA (the MMA's M)
 constexpr int FTHREADS = 256;
-constexpr uint32_t F_ACT_BYTES = FROWS * FACT_K * 2;   // 64 KB per row tile
-constexpr uint32_t F_W_BYTES = 256 * TBK * 2;          // 32 KB per weight stage
-constexpr uint32_t F_SMEM = FTILES * F_ACT_BYTES + 2 * F_W_BYTES + 64 + 1024;
+constexpr uint32_t F_ACT_BYTES = FROWS * FACT_K * 2;   // 64 KB
+constexpr uint32_t F_W_BYTES = 256 * TBK * 2;          // 32 KB
+constexpr uint32_t F_BIAS_BYTES = 2 * 256 * 4;         // this layer's and the next one's
+constexpr uint32_t F_SMEM = F_ACT_BYTES + F_W_BYTES + F_BIAS_BYTES + 64 + 1024;
+static_assert(2 * (F_SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
 
 __device__ __forceinline__ uint32_t act_off(int r, int k) {
   return (uint32_t)(((((r >> 3) * (FACT_K / 8)) + (k >> 3)) << 7) + ((r & 7) << 4) + ((k & 7) << 1));
@@ -368,39 +376,50 @@ __device__ __forceinline__ void store_w(uint8_t* s, const WChunk& c, int N) {
   }
 }
 
-__global__ void __launch_bounds__(FTHREADS, 1) mlp_fused_infer(FusedArgs a) {
+// The rows' inputs (FP32 [n][in], in <= 64) as BF16 columns 0..63 of the activation tile.
+__device__ __forceinline__ void stage_inputs(uint8_t* act, const float* x, long long m0, long long n,
+                                             int in) {
+#pragma unroll
+  for (int it = 0; it < FROWS * 8 / FTHREADS; ++it) {
+    const int q = threadIdx.x + it * FTHREADS, r = q & (FROWS - 1), k = (q / FROWS) * 8;
+    __nv_bfloat16 h[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      h[u] = __float2bfloat16_rn(m0 + r < n && k + u < in ? x[(m0 + r) * in + k + u] : 0.0f);
+    uint4 w;
+    memcpy(&w, h, 16);
+    *reinterpret_cast<uint4*>(act + act_off(r, k)) = w;
+  }
+}
+
+// Persistent: CTA b takes tiles b, b + gridDim.x, ... of the members' row blocks (member-major).
+// Two CTAs that start together run in step and wait for their products together; over many tiles
+// they drift apart until one's products run under the other's epilogue.
+__global__ void __launch_bounds__(FTHREADS, 2) mlp_fused_infer(const __grid_constant__ FusedArgs a,
+                                                               int nblk, int ntiles) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                            ~static_cast<uintptr_t>(1023));
-  uint8_t* act = sm;  // [FTILES][F_ACT_BYTES]
-  uint8_t* sW = sm + FTILES * F_ACT_BYTES;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sW + 2 * F_W_BYTES);
+  uint8_t* act = sm;
+  uint8_t* sW = sm + F_ACT_BYTES;
+  float* sBias = reinterpret_cast<float*>(sW + F_W_BYTES);  // [2][256]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sW + F_W_BYTES + F_BIAS_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int e = blockIdx.y;
-  const long long m0 = (long long)blockIdx.x * (FROWS * FTILES);
-  const __nv_bfloat16* wbf = a.wbf + e * a.P;
-  const float* prm = a.params + e * a.P;
-
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 256 * FTILES);
+    tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
   if (tid == 0) {
     mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
     fence_mbar_init();
   }
-  // inputs (FP32 [n][in], in <= 64) -> BF16 columns 0..63 of the activation tile
-  for (int q = tid; q < FTILES * FROWS * 64; q += FTHREADS) {
-    const int r = q >> 6, k = q & 63;  // r: row of the CTA, tile r / FROWS
-    const long long row = m0 + r;
-    float v = 0.0f;
-    if (row < a.n && k < a.dims[0]) v = a.x[row * a.dims[0] + k];
-    *reinterpret_cast<__nv_bfloat16*>(act + (r / FROWS) * F_ACT_BYTES + act_off(r % FROWS, k)) =
-        __float2bfloat16_rn(v);
-  }
+  int tile = (int)blockIdx.x;
+  int e = tile / nblk;
+  long long m0 = (long long)(tile - e * nblk) * FROWS;
+  stage_inputs(act, a.x, m0, a.n, a.dims[0]);
+  if (tid < a.dims[1]) sBias[tid] = a.params[e * a.P + a.b_off[0] + tid];
   fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -408,98 +427,109 @@ __global__ void __launch_bounds__(FTHREADS, 1) mlp_fused_infer(FusedArgs a) {
   const uint32_t tmem = *tmem_slot;
 
   WChunk pre;
-  load_w(pre, wbf + a.w_off[0], a.dims[1], a.dims[0], 0);
-  int g = 0;  // weight chunks committed so far; stage = g & 1
+  load_w(pre, a.wbf + e * a.P + a.w_off[0], a.dims[1], a.dims[0], 0);
+  int g = 0;   // weight chunks committed so far
+  int bp = 0;  // which half of sBias holds this layer's biases
   bool failed = false;
-  for (int l = 0; l < a.L && !failed; ++l) {
-    const int K = a.dims[l], N = a.dims[l + 1];
-    const int nch = (K + TBK - 1) / TBK;
-    for (int c = 0; c < nch; ++c) {
-      const int s = g & 1;
-      bool bad = false;
-      if (g >= 2 && !mbar_wait_bounded(&bar[s], ((g - 2) >> 1) & 1, kTcWaitLimit)) {
-        bad = true;
-        atomicExch(a.err, 1);
+  while (tile < ntiles && !failed) {
+    const int next = tile + (int)gridDim.x;
+    const int e2 = next < ntiles ? next / nblk : e;  // the next tile (of the last one: any weights)
+    for (int l = 0; l < a.L; ++l) {
+      const int K = a.dims[l], N = a.dims[l + 1];
+      const int nch = (K + TBK - 1) / TBK;
+      const bool last = l + 1 == a.L;
+      const int en = last ? e2 : e, ln = last ? 0 : l + 1;  // the layer after this one
+      for (int c = 0; c < nch; ++c) {
+        bool bad = false;
+        if (c > 0 && !mbar_wait_bounded(bar, (g - 1) & 1, kTcWaitLimit)) {  // (c = 0: waited below)
+          bad = true;
+          atomicExch(a.err, 1);
+        }
+        if (!bad) store_w(sW, pre, N);
+        fence_proxy_async_smem();
+        if (__syncthreads_or(bad)) {
+          failed = true;
+          break;
+        }
+        if (tid == 0) {
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(act), b0 = smem_u32(sW);
+#pragma unroll
+          for (int j = 0; j < TBK / 16; ++j)
+            umma_bf16(tmem, smem_desc_sbo(a0 + (uint32_t)(c * 8 + 2 * j) * 128u, FACT_K / 8 * 128),
+                      smem_desc_sbo(b0 + (uint32_t)j * 256u, TBK / 8 * 128), instr_desc_n(N),
+                      (c > 0 || j > 0) ? 1u : 0u);
+          umma_commit(bar);
+        }
+        ++g;
+        if (c + 1 < nch)
+          load_w(pre, a.wbf + e * a.P + a.w_off[l], N, K, (c + 1) * TBK);
+        else
+          load_w(pre, a.wbf + en * a.P + a.w_off[ln], a.dims[ln + 1], a.dims[ln], 0);
       }
-      if (!bad) store_w(sW + s * F_W_BYTES, pre, N);
-      fence_proxy_async_smem();
-      if (__syncthreads_or(bad)) {
+      if (failed) break;
+      // the next layer's biases: read after the barriers below
+      if (tid < a.dims[ln + 1]) sBias[(bp ^ 1) * 256 + tid] = a.params[en * a.P + a.b_off[ln] + tid];
+      bool late = !mbar_wait_bounded(bar, (g - 1) & 1, kTcWaitLimit);
+      if (late) atomicExch(a.err, 1);
+      if (__syncthreads_or(late)) {
         failed = true;
         break;
       }
-      if (c + 1 < nch)
-        load_w(pre, wbf + a.w_off[l], N, K, (c + 1) * TBK);
-      else if (l + 1 < a.L)
-        load_w(pre, wbf + a.w_off[l + 1], a.dims[l + 2], a.dims[l + 1], 0);
-      if (tid == 0) {
-        tc_fence_after();
-        const uint32_t b0 = smem_u32(sW + s * F_W_BYTES);
-#pragma unroll
-        for (int t = 0; t < FTILES; ++t) {
-          const uint32_t a0 = smem_u32(act + t * F_ACT_BYTES);
-#pragma unroll
-          for (int j = 0; j < TBK / 16; ++j)
-            umma_bf16(tmem + (uint32_t)(t * 256), smem_desc_sbo(a0 + (uint32_t)(c * 8 + 2 * j) * 128u,
-                                                                 FACT_K / 8 * 128),
-                      smem_desc_sbo(b0 + (uint32_t)j * 256u, TBK / 8 * 128), instr_desc_n(N),
-                      (c > 0 || j > 0) ? 1u : 0u);
-        }
-        umma_commit(&bar[s]);
-      }
-      ++g;
-    }
-    if (failed) break;
-    bool late = !mbar_wait_bounded(&bar[(g - 1) & 1], ((g - 1) >> 1) & 1, kTcWaitLimit);
-    if (late) atomicExch(a.err, 1);
-    if (__syncthreads_or(late)) {
-      failed = true;
-      break;
-    }
-    tc_fence_after();
-    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (rows of its tile) of tile w / 4
-    const int q4 = warp & 3, t = warp >> 2;
-    const int r = q4 * 32 + lane;
-    const long long row = m0 + t * FROWS + r;
-    uint8_t* tact = act + t * F_ACT_BYTES;
-    const float* bias = prm + a.b_off[l];
-    const bool last = l + 1 == a.L;
+      tc_fence_after();
+      // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (its rows)
+      const int q4 = warp & 3;
+      const int r = q4 * 32 + lane;
+      const long long row = m0 + r;
+      const float* bias = sBias + bp * 256;
+      if (last && next < ntiles)  // the products are done with the activations
+        stage_inputs(act, a.x, (long long)(next - e2 * nblk) * FROWS, a.n, a.dims[0]);
 #pragma unroll 1
-    for (int c0 = 0; c0 < N; c0 += 32) {
-      uint32_t v[32];
-      tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(t * 256 + c0), v);
-      tmem_wait_ld();
-      if (!last) {
+      for (int c0 = (warp >> 2) * 32; c0 < N; c0 += 64) {
+        uint32_t v[32];
+        tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)c0, v);
+        tmem_wait_ld();
+        if (!last) {
 #pragma unroll
-        for (int q = 0; q < 32; q += 8) {
-          __nv_bfloat16 h[8];
+          for (int q = 0; q < 32; q += 8) {
+            float b[8];
+            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(bias + c0 + q);
+            *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(bias + c0 + q + 4);
+            __nv_bfloat16 h[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            h[u] = __float2bfloat16_rn(gelu(__uint_as_float(v[q + u]) + bias[c0 + q + u]));
-          uint4 w;
-          memcpy(&w, h, 16);
-          *reinterpret_cast<uint4*>(tact + act_off(r, c0 + q)) = w;
+            for (int u = 0; u < 8; ++u)
+              h[u] = __float2bfloat16_rn(gelu(__uint_as_float(v[q + u]) + b[u]));
+            uint4 w;
+            memcpy(&w, h, 16);
+            *reinterpret_cast<uint4*>(act + act_off(r, c0 + q)) = w;
+          }
+        } else if (row < a.n) {
+          float* o = a.out + e * a.out_stride + row * N + c0;
+#pragma unroll
+          for (int q = 0; q < 32; q += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(bias + c0 + q);
+            *reinterpret_cast<float4*>(o + q) =
+                make_float4(__uint_as_float(v[q]) + b.x, __uint_as_float(v[q + 1]) + b.y,
+                            __uint_as_float(v[q + 2]) + b.z, __uint_as_float(v[q + 3]) + b.w);
+          }
         }
-      } else if (row < a.n) {
-        float* o = a.out + e * a.out_stride + row * N + c0;
-#pragma unroll
-        for (int q = 0; q < 32; q += 4)
-          *reinterpret_cast<float4*>(o + q) =
-              make_float4(__uint_as_float(v[q]) + bias[c0 + q], __uint_as_float(v[q + 1]) + bias[c0 + q + 1],
-                          __uint_as_float(v[q + 2]) + bias[c0 + q + 2],
-                          __uint_as_float(v[q + 3]) + bias[c0 + q + 3]);
       }
+      fence_proxy_async_smem();  // the new activations are the next MMAs' operand
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      bp ^= 1;
     }
-    fence_proxy_async_smem();  // the new activations are the next MMAs' operand
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    tile = next;
+    e = e2;
+    m0 = (long long)(next - e2 * nblk) * FROWS;
   }
   if (failed && g > 0) {  // let what was issued finish before the accumulator is released
-    (void)mbar_wait_bounded(&bar[(g - 1) & 1], ((g - 1) >> 1) & 1, kTcWaitLimit);
+    (void)mbar_wait_bounded(bar, (g - 1) & 1, kTcWaitLimit);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256 * FTILES);
+  if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
 }  // namespace
@@ -549,8 +579,12 @@ cudaError_t launch_mlp_fused(const FusedArgs& a, int members, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     set_on.fetch_or(bit);
   }
-  const dim3 grid((unsigned)((a.n + FROWS * FTILES - 1) / (FROWS * FTILES)), (unsigned)members);
-  mlp_fused_infer<<<grid, FTHREADS, F_SMEM, st>>>(a);
+  int nsm = 0;
+  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  const long long nblk = (a.n + FROWS - 1) / FROWS, ntiles = nblk * members;
+  if (ntiles > 0x7fffffffLL - 2 * nsm) return cudaErrorInvalidValue;
+  mlp_fused_infer<<<(unsigned)std::min<long long>(ntiles, 2 * nsm), FTHREADS, F_SMEM, st>>>(
+      a, (int)nblk, (int)ntiles);
   return cudaGetLastError();
 }
 
