@@ -163,15 +163,14 @@ __device__ __forceinline__ void h_cell(const Grid& g, const FieldPtrs& Fi, const
 // that touch an x layer (XL) are marched by blocks of their own: no warp runs the x-layer code
 // for a few of its lanes.  The y layers are uniform along a row, the z layers along a plane.
 //
-// Bound: memory latency at the occupancy the registers allow (38 bytes per cell and half step
-// plus the layers' psi).  So all loads of a plane are issued before its first store (a psi load
-// behind another psi array's store would wait for it), and the pointers stay in the constant
-// bank (kernel parameters) instead of registers.  B200, both half steps: 32 grids of 96^3 with 8
-// layer cells 0.61 ms a step (46 Gcell-updates/s; one thread per cell without a march 1.57 ms),
-// 256^3 with 10 layer cells 0.30 ms (55 Gcell-updates/s; 0.52 ms).  Four cells per thread (128
-// registers, 12 warps per SM instead of 20) took 0.74 ms and 0.33 ms.  Stepping the batch group
-// by group, each group small enough for the L2 cache, took longer (0.69 ms): what is missing
-// are loads in flight, not bandwidth.
+// Bound: memory (38 bytes per cell and half step plus the layers' psi) off the layers, latency in
+// them.  The pointers stay in the constant bank (kernel parameters) instead of registers; psi is
+// loaded where it is used, one axis after the other: that makes a chain of the layers' loads but
+// leaves 64 registers and 32 warps per SM, where loading everything first needs 80.  B200, both half
+// steps: 32 grids of 96^3 with 8 layer cells 0.55 ms a step (51 Gcell-updates/s; one thread per
+// cell without a march 1.57 ms; all loads first 0.58), 256^3 with 10 layer cells 0.28 ms (59; 0.52;
+// 0.30).  Four cells per thread (128 registers, 12 warps) took 0.74 and 0.33 ms; loading a plane
+// ahead, prefetching into L2, and stepping a batch in groups that fit the L2 cache gained nothing.
 constexpr int V = kCpmlV;
 constexpr int kHalfThreads = 128;
 
@@ -283,8 +282,6 @@ __device__ __forceinline__ void march_row(const CpmlHot& h, const CpmlSim& s, lo
     float* const d2 = h.F.f[H ? 5 : 2] + base;
     if (jrow) {
       if (k >= 1 && k <= g.nz - 2) {
-        // Every load of the plane first: a psi load behind the store of another psi array would
-        // wait for it (they may alias as far as the compiler knows), one memory latency each.
         Cells f0 = ldv(d0 + o), f1 = ldv(d1 + o), f2 = ldv(d2 + o);
         const Cells v2 = ldv(s2 + o);
         const Cells n0 = ldv(n0p + o), n1 = ldv(n1p + o);
@@ -297,28 +294,7 @@ __device__ __forceinline__ void march_row(const CpmlHot& h, const CpmlSim& s, lo
         ushort2 id = {};
         if (h.mat) id = *reinterpret_cast<const ushort2*>(h.mat + base + o);
         const int zs = H ? Z.slot_h[k] : Z.slot_e[k];
-        Cells py2, py0, pz1, pz0;
-        Cells px2, px1;
-        const uint32_t oyp = (uint32_t)(i0 + g.nx * ys), ozp = (uint32_t)(i0 + g.nx * j);
-        const long long byp = (long long)g.nx * Y.S * k, bzp = (long long)g.nx * g.ny * zs;
-        const uint32_t oxp = (uint32_t)(xs + X.S * j);
-        const long long bxp = (long long)X.S * g.ny * k;
         float* const* psi = H ? h.P.psi_h : h.P.psi_e;
-        if (ys >= 0) {
-          py2 = ld_psi(psi[H ? 1 : 0] + byp + oyp, vec, upd);
-          py0 = ld_psi(psi[H ? 4 : 5] + byp + oyp, vec, upd);
-        }
-        if (zs >= 0) {
-          pz1 = ld_psi(psi[H ? 0 : 1] + bzp + ozp, vec, upd);
-          pz0 = ld_psi(psi[H ? 3 : 2] + bzp + ozp, vec, upd);
-        }
-        if (XL) {
-#pragma unroll
-          for (int e = 0; e < V; ++e) {
-            px2.v[e] = xin[e] ? psi[H ? 2 : 3][bxp + oxp + e] : 0.0f;
-            px1.v[e] = xin[e] ? psi[H ? 5 : 4][bxp + oxp + e] : 0.0f;
-          }
-        }
         // curl = (dy2 - dz1, dz0 - dx2, dx1 - dy0) for E, the negative for H
         Cells dy2 = H ? subv(y2, v2) : subv(v2, y2), dy0 = H ? subv(y0, c0) : subv(n0, y0);
         Cells dz1 = subv(n1, c1), dz0 = subv(n0, c0), dx2, dx1;
@@ -333,29 +309,41 @@ __device__ __forceinline__ void march_row(const CpmlHot& h, const CpmlSim& s, lo
           }
         }
         if (ys >= 0) {
-          stretch(dy2, yb, ya, yi, py2, upd);
-          stretch(dy0, yb, ya, yi, py0, upd);
-          st_psi(psi[H ? 1 : 0] + byp + oyp, py2, vec, upd);
-          st_psi(psi[H ? 4 : 5] + byp + oyp, py0, vec, upd);
+          float* const a2 = psi[H ? 1 : 0] + (long long)g.nx * Y.S * k + (uint32_t)(i0 + g.nx * ys);
+          float* const a0 = psi[H ? 4 : 5] + (long long)g.nx * Y.S * k + (uint32_t)(i0 + g.nx * ys);
+          Cells p2 = ld_psi(a2, vec, upd), p0 = ld_psi(a0, vec, upd);
+          stretch(dy2, yb, ya, yi, p2, upd);
+          stretch(dy0, yb, ya, yi, p0, upd);
+          st_psi(a2, p2, vec, upd);
+          st_psi(a0, p0, vec, upd);
         }
         if (zs >= 0) {
           const float b = H ? Z.bh[k] : Z.be[k], a = H ? Z.ah[k] : Z.ae[k];
           const float ik = H ? Z.ikh[k] : Z.ike[k];
-          stretch(dz1, b, a, ik, pz1, upd);
-          stretch(dz0, b, a, ik, pz0, upd);
-          st_psi(psi[H ? 0 : 1] + bzp + ozp, pz1, vec, upd);
-          st_psi(psi[H ? 3 : 2] + bzp + ozp, pz0, vec, upd);
+          float* const a1 = psi[H ? 0 : 1] + (long long)g.nx * g.ny * zs + (uint32_t)(i0 + g.nx * j);
+          float* const a0 = psi[H ? 3 : 2] + (long long)g.nx * g.ny * zs + (uint32_t)(i0 + g.nx * j);
+          Cells p1 = ld_psi(a1, vec, upd), p0 = ld_psi(a0, vec, upd);
+          stretch(dz1, b, a, ik, p1, upd);
+          stretch(dz0, b, a, ik, p0, upd);
+          st_psi(a1, p1, vec, upd);
+          st_psi(a0, p0, vec, upd);
         }
         if (XL) {
+          float* const a2 = psi[H ? 2 : 3] + (long long)X.S * g.ny * k + (xs + X.S * j);
+          float* const a1 = psi[H ? 5 : 4] + (long long)X.S * g.ny * k + (xs + X.S * j);
+          Cells p2, p1;
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            p2.v[e] = xin[e] ? a2[e] : 0.0f;
+            p1.v[e] = xin[e] ? a1[e] : 0.0f;
+          }
 #pragma unroll
           for (int e = 0; e < V; ++e)
             if (xin[e]) {
-              px2.v[e] = add(mul(xb[e], px2.v[e]), mul(xa[e], dx2.v[e]));
-              px1.v[e] = add(mul(xb[e], px1.v[e]), mul(xa[e], dx1.v[e]));
-              dx2.v[e] = add(mul(dx2.v[e], xi[e]), px2.v[e]);
-              dx1.v[e] = add(mul(dx1.v[e], xi[e]), px1.v[e]);
-              psi[H ? 2 : 3][bxp + oxp + e] = px2.v[e];
-              psi[H ? 5 : 4][bxp + oxp + e] = px1.v[e];
+              a2[e] = p2.v[e] = add(mul(xb[e], p2.v[e]), mul(xa[e], dx2.v[e]));
+              a1[e] = p1.v[e] = add(mul(xb[e], p1.v[e]), mul(xa[e], dx1.v[e]));
+              dx2.v[e] = add(mul(dx2.v[e], xi[e]), p2.v[e]);
+              dx1.v[e] = add(mul(dx1.v[e], xi[e]), p1.v[e]);
             }
         }
         // E: (dyHz - dzHy, dzHx - dxHz, dxHy - dyHx); H: (dzEy - dyEz, dxEz - dzEx, dyEx - dxEy)
@@ -452,7 +440,7 @@ __device__ __forceinline__ void half_block(const CpmlHot& h, const CpmlSim& s, l
 
 // One grid (arguments in the parameters): blockIdx.x = cells, blockIdx.y = z-chunk of zc planes.
 template <bool H>
-__global__ void __launch_bounds__(kHalfThreads, 6) cpml_half(const __grid_constant__ CpmlHot h,
+__global__ void __launch_bounds__(kHalfThreads, 8) cpml_half(const __grid_constant__ CpmlHot h,
                                                           const __grid_constant__ CpmlSim s,
                                                           long long t, int zc) {
   const int k0 = (int)blockIdx.y * zc;
@@ -461,7 +449,7 @@ __global__ void __launch_bounds__(kHalfThreads, 6) cpml_half(const __grid_consta
 
 // A group of grids of a batch: blockIdx.z = grid of the group.
 template <bool H>
-__global__ void __launch_bounds__(kHalfThreads, 6)
+__global__ void __launch_bounds__(kHalfThreads, 8)
     cpml_half_batch(const __grid_constant__ CpmlGroup grp, const CpmlSim* __restrict__ sims,
                     long long t_offset, int zc) {
   const CpmlHot& h = grp.h[blockIdx.z];
