@@ -28,6 +28,7 @@ using fdtd::Material;
 namespace {
 
 constexpr int kMaxMaterials = 65536;
+constexpr size_t kKeepEps = 64u << 20;
 constexpr double kPiD = 3.14159265358979323846;
 
 enum CoefMode { kCoefNone = 0, kCoefMaterial = 1, kCoefPerCell = 2 };
@@ -120,6 +121,10 @@ struct fdtd_handle {
   Material* table = nullptr;
   int nmat = 0;
   void* scratch = nullptr;
+  // fdtd_set_permittivity: stretch profiles and permittivity, kept between calls (the permittivity
+  // up to kKeepEps bytes)
+  float2* d_prof = nullptr;
+  float* d_eps = nullptr;
   fdtd::SourceDev src[fdtd::kMaxSources] = {};
   int nsrc = 0;
   float* d_wave = nullptr;
@@ -393,7 +398,9 @@ fdtd::TiledArgs make_tiled_args(fdtd_handle* h, const fdtd::TiledConfig& c, long
 std::vector<fdtd::TiledConfig> candidates(const fdtd_handle* h) {
   std::vector<fdtd::TiledConfig> out;
   std::vector<int> blts = {1, 2, 3, 4, 5, 6}, rows_l = {8, 16, 20, 24, 32, 48};
-  std::vector<int> zc = {1, 2, 4, 8};
+  // Fine steps: the last wave of CTAs is nearly empty or nearly full depending on the count (256^3,
+  // 20-row tiles: 8 chunks fill 4.3 waves, 7 fill 3.8 and waste less on warm-up planes).
+  std::vector<int> zc = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 16};
   // kernel families: 0 one cell per thread (32-wide rows), 1 x-pairs in 64-wide rows,
   // 2 x-pairs in 32-wide rows (two per warp)
   std::vector<int> fams = {0, 1, 2};
@@ -437,8 +444,8 @@ std::vector<fdtd::TiledConfig> candidates(const fdtd_handle* h) {
   return out;
 }
 
-// Times every candidate on the current field set (source set -> scratch destination; sources
-// and monitors off, so the simulation state is not changed) and keeps the fastest per step.
+// Times every candidate on the current field set (source set -> scratch destination; monitors
+// off, so the simulation state is not changed) and keeps the fastest per step.
 fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
   const auto key = std::make_tuple(h->g.nx, h->g.ny, h->g.nz,
                                    (h->cpml_on ? 10000000000LL : 0LL) +
@@ -470,7 +477,8 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
       -> fdtd_status {
     fdtd_status s = ensure_maps(h, c);
     if (s != FDTD_OK) return s;
-    const fdtd::TiledArgs a = make_tiled_args(h, c, 0, false);
+    fdtd::TiledArgs a = make_tiled_args(h, c, 0, false);
+    a.S = make_sources(h);  // on a small grid the tile with the source ends last
     CUDA_TRY(h, launch_any(c, a, h->g, st));
     for (int pass = 0; pass < 2; ++pass) {
       CUDA_TRY(h, cudaEventRecord(e0, st));
@@ -584,6 +592,8 @@ void free_all(fdtd_handle* h) {
   cudaFree(h->mat);
   cudaFree(h->table);
   cudaFree(h->scratch);
+  cudaFree(h->d_prof);
+  cudaFree(h->d_eps);
   cudaFree(h->d_wave);
   cudaFree(h->d_err);
   cudaFree(h->ublk);
@@ -1135,27 +1145,28 @@ fdtd_status fdtd_set_permittivity(fdtd_handle* h, const float* eps_re, int32_t t
                                  stretch_profile(h->g.ny, t_pml, sigma_max, omega0),
                                  stretch_profile(h->g.nz, t_pml, sigma_max, omega0)};
   const size_t n = (size_t)h->g.nx * h->g.ny * h->g.nz;
-  float2* d_prof = nullptr;
-  float* d_eps = nullptr;
   const size_t np = prof[0].size() + prof[1].size() + prof[2].size();
-  CUDA_TRY(h, cudaMalloc(&d_prof, np * sizeof(float2)));
-  CUDA_TRY(h, cudaMemcpyAsync(d_prof, prof[0].data(), prof[0].size() * 8, cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(d_prof + prof[0].size(), prof[1].data(), prof[1].size() * 8,
-                              cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(d_prof + prof[0].size() + prof[1].size(), prof[2].data(),
-                              prof[2].size() * 8, cudaMemcpyHostToDevice, h->stream));
+  if (!h->d_prof) CUDA_TRY(h, cudaMalloc(&h->d_prof, np * sizeof(float2)));
+  float2* const d_prof = h->d_prof;
+  std::vector<float2> all;  // one copy for the three axes
+  for (const auto& p : prof) all.insert(all.end(), p.begin(), p.end());
+  CUDA_TRY(h, cudaMemcpyAsync(d_prof, all.data(), np * sizeof(float2), cudaMemcpyHostToDevice,
+                              h->stream));
   if (eps_re) {
-    CUDA_TRY(h, cudaMalloc(&d_eps, n * sizeof(float)));
-    CUDA_TRY(h, cudaMemcpyAsync(d_eps, eps_re, n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    if (!h->d_eps) CUDA_TRY(h, cudaMalloc(&h->d_eps, n * sizeof(float)));
+    CUDA_TRY(h, cudaMemcpyAsync(h->d_eps, eps_re, n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   }
   fdtd::Coef12Out out;
   for (int a = 0; a < 12; ++a) out.c[a] = h->coef[a];
-  CUDA_TRY(h, fdtd::build_coefficients(h->g, d_eps, d_prof, d_prof + prof[0].size(),
+  CUDA_TRY(h, fdtd::build_coefficients(h->g, eps_re ? h->d_eps : nullptr, d_prof,
+                                       d_prof + prof[0].size(),
                                        d_prof + prof[0].size() + prof[1].size(), omega0, dt, dx,
                                        out, h->stream));
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  cudaFree(d_prof);
-  cudaFree(d_eps);
+  if (n * sizeof(float) > kKeepEps && h->d_eps) {
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    cudaFree(h->d_eps);
+    h->d_eps = nullptr;
+  }
   return compress_coefficients(h);
 }
 

@@ -722,8 +722,9 @@ __global__ void __launch_bounds__(TY * W / 2, (batch_min_blocks<TY, W>()))
 template <typename S, int B, int TY, int MINB, int W = 64, typename SH = S>
 cudaError_t launch_one2(const TiledArgs& a, dim3 grid, cudaStream_t st) {
   using K = Tiled2<S, B, TY, W, SH>;
-  cudaError_t e = cudaFuncSetAttribute(fdtd_tiled2<S, B, TY, MINB, W, SH>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::SMEM);
+  static std::atomic<unsigned long long> done{0};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(&fdtd_tiled2<S, B, TY, MINB, W, SH>),
+                             K::SMEM, done);
   if (e != cudaSuccess) return e;
   fdtd_tiled2<S, B, TY, MINB, W, SH><<<grid, dim3(32, K::THREADS / 32), K::SMEM, st>>>(a);
   return cudaGetLastError();
@@ -732,8 +733,9 @@ cudaError_t launch_one2(const TiledArgs& a, dim3 grid, cudaStream_t st) {
 template <typename S, int B, int TY, int W = 64, typename SH = S>
 cudaError_t launch_batch_one(const BatchArgs& b, int ctas, cudaStream_t st) {
   using K = Tiled2<S, B, TY, W, SH>;
-  cudaError_t e = cudaFuncSetAttribute(fdtd_tiled2_batch<S, B, TY, W, SH>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::SMEM);
+  static std::atomic<unsigned long long> done{0};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(&fdtd_tiled2_batch<S, B, TY, W, SH>),
+                             K::SMEM, done);
   if (e != cudaSuccess) return e;
   fdtd_tiled2_batch<S, B, TY, W, SH><<<ctas, dim3(32, K::THREADS / 32), K::SMEM, st>>>(b);
   return cudaGetLastError();
