@@ -220,6 +220,13 @@ fdtd_status fail(fdtd_handle* h, fdtd_status s, const char* fmt, ...) {
                   "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
   } while (0)
 
+// Uploads of pageable host memory and clears, complete when they return.  (The handle's streams do
+// not wait for the legacy stream, on which cudaMemcpy may return before its data has arrived.)
+cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 struct DeviceGuard {
   int prev = -1;
   explicit DeviceGuard(int dev) {
@@ -346,7 +353,7 @@ fdtd_status ensure_tables(fdtd_handle* h, long long upto) {
     double2* d = nullptr;
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     CUDA_TRY(h, cudaMalloc(&d, host.size() * sizeof(double2)));
-    CUDA_TRY(h, cudaMemcpy(d, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice));
+    CUDA_TRY(h, upload(d, host.data(), host.size() * sizeof(double2), h->stream));
     if (mh.tab) cudaFree(mh.tab);
     mh.tab = d;
     mh.tab_cap = cap;
@@ -563,7 +570,7 @@ fdtd_status check_device_error(fdtd_handle* h) {
   int e = 0;
   CUDA_TRY(h, cudaMemcpy(&e, h->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e != fdtd::kErrNone) {
-    cudaMemset(h->d_err, 0, sizeof(int));
+    cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
     if (e & fdtd::kErrTimeout)
       return fail(h, FDTD_ERR_DEVICE_TIMEOUT,
                   "a device-side bounded wait expired (error word %d); results are invalid", e);
@@ -857,8 +864,8 @@ const int* tile_order(fdtd_handle* h, const fdtd::TiledConfig& c) {
     if (cudaMalloc(&h->d_order, (size_t)ntile * sizeof(int)) != cudaSuccess) return nullptr;
     h->order_cap = ntile;
   }
-  if (cudaMemcpy(h->d_order, h->order_host.data(), (size_t)ntile * sizeof(int),
-                 cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload(h->d_order, h->order_host.data(), (size_t)ntile * sizeof(int), h->stream) !=
+      cudaSuccess)
     return nullptr;
   return h->d_order;
 }
@@ -931,7 +938,7 @@ fdtd_status cpml_region_blocks(fdtd_handle* h, int r, std::pair<int4*, int>* out
   }
   int4* d = nullptr;
   CUDA_TRY(h, cudaMalloc(&d, std::max<size_t>(v.size(), 1) * sizeof(int4)));
-  const cudaError_t e = cudaMemcpy(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice);
+  const cudaError_t e = upload(d, v.data(), v.size() * sizeof(int4), h->stream);
   if (e != cudaSuccess) {
     cudaFree(d);
     return fail(h, FDTD_ERR_CUDA, "CPML block list upload failed: %s", cudaGetErrorString(e));
@@ -1216,7 +1223,7 @@ fdtd_status fdtd_set_sources(fdtd_handle* h, const fdtd_source* sources, int32_t
   if (nsrc > 0) {
     const size_t bytes = (size_t)nsrc * T_wave * sizeof(float);
     CUDA_TRY(h, cudaMalloc(&h->d_wave, bytes));
-    CUDA_TRY(h, cudaMemcpy(h->d_wave, waveforms, bytes, cudaMemcpyHostToDevice));
+    CUDA_TRY(h, upload(h->d_wave, waveforms, bytes, h->stream));
   }
   for (int n = 0; n < nsrc; ++n) {
     h->src[n].comp = sources[n].component;
@@ -1729,10 +1736,9 @@ fdtd_status fdtd_set_cpml(fdtd_handle* h, const fdtd_cpml_desc* d) {
       cpml_profile(*d, n[a], lo, hi, (double)h->desc.dx, k == 1, &sl, &pr[0], &pr[1], &pr[2]);
       int* d_slot = reinterpret_cast<int*>(base + off);
       float* d_f = reinterpret_cast<float*>(base + off + (size_t)n[a] * 4);
-      CUDA_TRY(h, cudaMemcpy(d_slot, sl.data(), (size_t)n[a] * 4, cudaMemcpyHostToDevice));
+      CUDA_TRY(h, upload(d_slot, sl.data(), (size_t)n[a] * 4, h->stream));
       for (int q = 0; q < 3; ++q)
-        CUDA_TRY(h, cudaMemcpy(d_f + (size_t)q * n[a], pr[q].data(), (size_t)n[a] * 4,
-                               cudaMemcpyHostToDevice));
+        CUDA_TRY(h, upload(d_f + (size_t)q * n[a], pr[q].data(), (size_t)n[a] * 4, h->stream));
       if (k == 0) {
         ax.slot_e = d_slot;
         ax.be = d_f;
@@ -1753,9 +1759,10 @@ fdtd_status fdtd_set_cpml(fdtd_handle* h, const fdtd_cpml_desc* d) {
       fdtd_set_cpml(h, nullptr);
       return fail(h, FDTD_ERR_OOM, "CPML psi allocation failed");
     }
-    CUDA_TRY(h, cudaMemset(h->cpml_psi[q], 0, pb));
+    CUDA_TRY(h, cudaMemsetAsync(h->cpml_psi[q], 0, pb, h->stream));
     (q < 6 ? h->cpml_dev.psi_e[q] : h->cpml_dev.psi_h[q - 6]) = h->cpml_psi[q];
   }
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   // positions whose updates involve no layer, per axis (the shell companion's inner box)
   for (int a = 0; a < 3; ++a) {
     int lo = 0, hi = n[a];
@@ -1820,7 +1827,7 @@ fdtd_status fdtd_set_cpml_psi(fdtd_handle* h, int32_t q, const void* host_in) {
   if (!h || !host_in || q < 0 || q > 11 || !h->cpml_on) return FDTD_ERR_INVALID_ARG;
   DeviceGuard dg(h->desc.device);
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  CUDA_TRY(h, cudaMemcpy(h->cpml_psi[q], host_in, cpml_psi_bytes(h, q), cudaMemcpyHostToDevice));
+  CUDA_TRY(h, upload(h->cpml_psi[q], host_in, cpml_psi_bytes(h, q), h->stream));
   return FDTD_OK;
 }
 
@@ -1954,7 +1961,7 @@ fdtd_status batch_items(fdtd_batch* b, const fdtd::TiledConfig& c, std::pair<int
   for (size_t i = 0; i < v.size(); ++i) host[i] = v[i].second;
   int4* d = nullptr;
   BCUDA(b, cudaMalloc(&d, host.size() * sizeof(int4)));
-  BCUDA(b, cudaMemcpy(d, host.data(), host.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  BCUDA(b, upload(d, host.data(), host.size() * sizeof(int4), b->stream));
   b->items[key] = {d, (int)host.size()};
   *out = b->items[key];
   return FDTD_OK;

@@ -409,7 +409,7 @@ fdtd_status check_after(fdtd_mlp* m) {
   if (cudaMemcpy(&w, m->d_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
     return mfail(m, FDTD_ERR_CUDA, "reading the device error word failed");
   if (w) {
-    cudaMemset(m->d_err, 0, sizeof(int));
+    cudaMemsetAsync(m->d_err, 0, sizeof(int), m->st);
     return mfail(m, FDTD_ERR_DEVICE_TIMEOUT,
                  "a bounded wait in a tensor-core GEMM expired; results are invalid");
   }
@@ -582,7 +582,7 @@ fdtd_status fdtd_mlp_create(const int32_t* dims, int32_t n_dims, int32_t members
       cudaMalloc(&m->adam_v, tot * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&m->wbf, tot * sizeof(__nv_bfloat16)) != cudaSuccess ||
       cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess ||
-      cudaMemset(m->d_err, 0, sizeof(int)) != cudaSuccess) {
+      cudaMemsetAsync(m->d_err, 0, sizeof(int), m->st) != cudaSuccess) {
     destroy(m);
     return FDTD_ERR_OOM;
   }
@@ -596,11 +596,13 @@ fdtd_status fdtd_mlp_create(const int32_t* dims, int32_t n_dims, int32_t members
       for (long long i = 0; i < (long long)dims[l] * dims[l + 1]; ++i) w[i] = nd(rng);
     }
   }
-  bool ok = cudaMemcpy(m->params, host.data(), tot * sizeof(float), cudaMemcpyHostToDevice) ==
-                cudaSuccess &&
-            cudaMemset(m->grads, 0, tot * sizeof(float)) == cudaSuccess &&
-            cudaMemset(m->adam_m, 0, tot * sizeof(float)) == cudaSuccess &&
-            cudaMemset(m->adam_v, 0, tot * sizeof(float)) == cudaSuccess;
+  // On the handle's own stream: it does not wait for the legacy stream, on which a copy of pageable
+  // memory may return before its data has arrived.
+  bool ok = cudaMemcpyAsync(m->params, host.data(), tot * sizeof(float), cudaMemcpyHostToDevice,
+                            m->st) == cudaSuccess &&
+            cudaMemsetAsync(m->grads, 0, tot * sizeof(float), m->st) == cudaSuccess &&
+            cudaMemsetAsync(m->adam_m, 0, tot * sizeof(float), m->st) == cudaSuccess &&
+            cudaMemsetAsync(m->adam_v, 0, tot * sizeof(float), m->st) == cudaSuccess;
   if (ok) {
     fdtd::mlp::to_bf16<<<fdtd::mlp::nblocks(tot), 256, 0, m->st>>>(tot, m->params, m->wbf);
     ok = cudaStreamSynchronize(m->st) == cudaSuccess;
@@ -651,7 +653,7 @@ fdtd_status fdtd_mlp_set_params(fdtd_mlp* m, const float* in) {
   MCUDA(m, cudaSetDevice(m->device));
   const long long tot = m->E * m->P;
   MCUDA(m, cudaStreamSynchronize(m->st));
-  MCUDA(m, cudaMemcpy(m->params, in, tot * sizeof(float), cudaMemcpyHostToDevice));
+  MCUDA(m, cudaMemcpyAsync(m->params, in, tot * sizeof(float), cudaMemcpyHostToDevice, m->st));
   fdtd::mlp::to_bf16<<<fdtd::mlp::nblocks(tot), 256, 0, m->st>>>(tot, m->params, m->wbf);
   MCUDA(m, cudaMemsetAsync(m->adam_m, 0, tot * sizeof(float), m->st));
   MCUDA(m, cudaMemsetAsync(m->adam_v, 0, tot * sizeof(float), m->st));
@@ -671,8 +673,9 @@ fdtd_status fdtd_mlp_set_data(fdtd_mlp* m, const float* x, const float* y, int64
   const int in = m->dims[0], out = m->dims[m->L];
   MCUDA(m, cudaMalloc(&m->X, n * in * sizeof(float)));
   MCUDA(m, cudaMalloc(&m->Y, n * out * sizeof(float)));
-  MCUDA(m, cudaMemcpy(m->X, x, n * in * sizeof(float), cudaMemcpyHostToDevice));
-  MCUDA(m, cudaMemcpy(m->Y, y, n * out * sizeof(float), cudaMemcpyHostToDevice));
+  MCUDA(m, cudaMemcpyAsync(m->X, x, n * in * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  MCUDA(m, cudaMemcpyAsync(m->Y, y, n * out * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  MCUDA(m, cudaStreamSynchronize(m->st));  // the caller may free x and y
   m->n = n;
   return FDTD_OK;
 }
