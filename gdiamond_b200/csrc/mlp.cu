@@ -294,6 +294,8 @@ struct fdtd_mlp {
   float* tgt = nullptr;                        // [E][cap][out]
   float* xin = nullptr;                        // FP32 input staging [cap][in]
   std::vector<__nv_bfloat16*> gl;  // train_epoch: gl[l] [E][cap][dims[l+1]], gradients of layer l
+  float* pred = nullptr;  // fused inference: every member's outputs of a chunk of rows
+  size_t pred_cap = 0;
   // training workspace, kept between calls: row order [E][n], summed losses, bias corrections
   int* perm = nullptr;
   float* dloss = nullptr;
@@ -491,6 +493,7 @@ void destroy(fdtd_mlp* m) {
   cudaFree(m->adam_v);
   cudaFree(m->wbf);
   cudaFree(m->d_err);
+  cudaFree(m->pred);
   cudaFree(m->perm);
   cudaFree(m->dloss);
   cudaFree(m->corr);
@@ -505,11 +508,18 @@ void destroy(fdtd_mlp* m) {
 fdtd_status predict_rows(fdtd_mlp* m, const float* x_dev, long long n, float* mean, float* sd,
                          float* per_member) {
   const int in = m->dims[0], out = m->dims[m->L];
-  const long long chunk = std::min<long long>(n, 65536);
-  fdtd_status s = ensure_cap(m, chunk);
-  if (s != FDTD_OK) return s;
   const bool fused = m->gemm_kind != FDTD_MLP_GEMM_MMA_SYNC && m->L <= fdtd::mlp::kFusedMaxLayers &&
                      fdtd::mlp::mlp_fused_supported(m->dims.data(), m->L);
+  // The fused kernel writes the outputs only (no activations of 65536 rows: 2 GB for the surrogate's
+  // network), so it takes longer chunks.
+  const long long chunk = std::min<long long>(n, fused ? 262144 : 65536);
+  fdtd_status s = FDTD_OK;
+  if (fused)
+    MCUDA(m, grow(m, &m->pred, &m->pred_cap, (size_t)m->E * chunk * out));
+  else if ((s = ensure_cap(m, chunk)) != FDTD_OK)
+    return s;
+  float* const y = fused ? m->pred : m->z[m->L - 1];  // [E][stride]
+  const long long stride = (fused ? chunk : m->cap) * out;
   for (long long r0 = 0; r0 < n; r0 += chunk) {
     const long long cnt = std::min<long long>(chunk, n - r0);
     if (fused) {  // every layer in one kernel: activations never leave the SM
@@ -525,8 +535,8 @@ fdtd_status predict_rows(fdtd_mlp* m, const float* x_dev, long long n, float* me
       fa.wbf = m->wbf;
       fa.params = m->params;
       fa.P = m->P;
-      fa.out = m->z[m->L - 1];
-      fa.out_stride = m->cap * out;
+      fa.out = y;
+      fa.out_stride = stride;
       fa.err = m->d_err;
       const cudaError_t le = fdtd::mlp::launch_mlp_fused(fa, m->E, m->st);
       if (le != cudaSuccess && m->launch_err == cudaSuccess) m->launch_err = le;
@@ -536,11 +546,11 @@ fdtd_status predict_rows(fdtd_mlp* m, const float* x_dev, long long n, float* me
       forward(m, (int)cnt, 0, /*keep_z=*/false);
     }
     fdtd::mlp::ens_stats<<<fdtd::mlp::nblocks(cnt * out), 256, 0, m->st>>>(
-        cnt * out, m->E, m->z[m->L - 1], m->cap * out, mean + r0 * out, sd + r0 * out);
+        cnt * out, m->E, y, stride, mean + r0 * out, sd + r0 * out);
     if (per_member)
       for (int e = 0; e < m->E; ++e)
         MCUDA(m, cudaMemcpyAsync(per_member + ((long long)e * n + r0) * out,
-                                 m->z[m->L - 1] + e * m->cap * out, cnt * out * sizeof(float),
+                                 y + e * stride, cnt * out * sizeof(float),
                                  cudaMemcpyDeviceToDevice, m->st));
   }
   MCUDA(m, cudaGetLastError());
