@@ -408,31 +408,59 @@ bool train_epoch_supported(const int* dims, int L, int batch) {
 
 namespace {
 
-// A member's cluster: 16 CTAs (more than the portable 8) while every member gets one at the same
-// time, 8 for larger ensembles.
+// Sets the kernel up on the current device, once; *ok: the device can hold a cluster of CTAS.
 template <int CTAS>
-cudaError_t launch_clusters(const TrainArgs& a, int members, cudaStream_t st) {
-  static std::atomic<unsigned long long> set_on{0};  // devices (bit per ordinal < 64) done
+cudaError_t set_up(bool* ok) {
+  static std::atomic<unsigned long long> done{0}, fits{0};  // a bit per device ordinal < 64
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (!(set_on.load() & bit) || !bit) {
-    e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSmem);
-    if (e == cudaSuccess && CTAS > 8)
-      e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    set_on.fetch_or(bit);
+  *ok = (fits.load() & bit) != 0;
+  if (bit && (done.load() & bit)) return cudaSuccess;
+  e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kSmem);
+  if (e == cudaSuccess && CTAS > 8)
+    e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = CTAS;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CTAS);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, train_epoch<CTAS>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
   }
-  train_epoch<CTAS><<<CTAS * members, kThreads, kSmem, st>>>(a);
-  return cudaGetLastError();
+  *ok = n > 0;
+  if (*ok) fits.fetch_or(bit);
+  done.fetch_or(bit);
+  return cudaSuccess;
 }
 
 }  // namespace
 
+// A member's cluster: 16 CTAs (more than the portable 8) for small ensembles, whose members then
+// all run at once, where the device has a GPC with 16 free SMs; 8 otherwise.
 cudaError_t launch_train_epoch(const TrainArgs& a, int members, cudaStream_t st) {
-  return members <= 4 ? launch_clusters<16>(a, members, st) : launch_clusters<8>(a, members, st);
+  bool ok = false;
+  cudaError_t e;
+  if (members <= 4) {
+    if ((e = set_up<16>(&ok)) != cudaSuccess) return e;
+    if (ok) {
+      train_epoch<16><<<16 * members, kThreads, kSmem, st>>>(a);
+      return cudaGetLastError();
+    }
+  }
+  if ((e = set_up<8>(&ok)) != cudaSuccess) return e;
+  train_epoch<8><<<8 * members, kThreads, kSmem, st>>>(a);
+  return cudaGetLastError();
 }
 
 }  // namespace mlp
