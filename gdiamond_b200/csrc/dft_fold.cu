@@ -11,9 +11,9 @@
 // a read-modify-write of 2 * nf doubles (1 KB at 32 frequencies), and the sums are read and
 // written once per window.
 //
-// A thread owns one plane cell and kFoldF frequencies: their sums stay in registers for the
-// whole window, the staged values of consecutive cells are coalesced, and the (cos, sin) table
-// row of each step is a broadcast.
+// A thread owns two plane cells and kFoldF frequencies: their sums stay in registers for the whole
+// window, the staged values of consecutive cells are coalesced, and each (cos, sin) pair of a
+// step, a broadcast load, serves both cells.  Bound: FP64 issue.
 #include <type_traits>
 
 #include "fdtd_kernels.cuh"
@@ -25,41 +25,53 @@ namespace {
 constexpr int kFoldThreads = 128;
 constexpr int kFoldF = 8;  // frequencies per thread
 
+constexpr int kFoldP = 2;  // plane cells per thread, kFoldThreads apart
+
 __device__ __forceinline__ void fold_monitor(const MonitorDev& m, const Grid& g, long long t0,
                                              int n) {
   const long long np = (long long)g.nx * g.ny;
-  const long long p = (long long)blockIdx.x * kFoldThreads + threadIdx.x;
+  const long long p0 = (long long)blockIdx.x * (kFoldThreads * kFoldP) + threadIdx.x;
   const int f0 = (int)blockIdx.y * kFoldF;
-  if (m.stage == nullptr || p >= np || f0 >= m.nf) return;
+  if (m.stage == nullptr || p0 >= np || f0 >= m.nf) return;
   const int nfc = min(kFoldF, m.nf - f0);
-  double re[kFoldF], im[kFoldF];
+  // a thread without a second cell folds its first one twice and stores it once
+  const bool two = p0 + kFoldThreads < np;
+  const long long p[kFoldP] = {p0, two ? p0 + kFoldThreads : p0};
+  double re[kFoldP][kFoldF], im[kFoldP][kFoldF];
 #pragma unroll
-  for (int q = 0; q < kFoldF; ++q) {
-    re[q] = q < nfc ? m.re[(long long)(f0 + q) * np + p] : 0.0;
-    im[q] = q < nfc ? m.im[(long long)(f0 + q) * np + p] : 0.0;
-  }
-  const float* st = m.stage + p;
+  for (int c = 0; c < kFoldP; ++c)
+#pragma unroll
+    for (int q = 0; q < kFoldF; ++q) {
+      re[c][q] = q < nfc ? m.re[(long long)(f0 + q) * np + p[c]] : 0.0;
+      im[c][q] = q < nfc ? m.im[(long long)(f0 + q) * np + p[c]] : 0.0;
+    }
+  const float* const st0 = m.stage + p[0];
+  const float* const st1 = m.stage + p[1];
   const double scale = m.scale;
   const int nf = m.nf;
   const double2* tab0 = m.tab + t0 * nf + f0;
   const int slot0 = (int)(t0 & (kDftSlots - 1));
   // x * 1.0 == x: without a scale two of the six operations per step and frequency fall away.
   auto window = [&](auto scaled, auto full) {
-#pragma unroll 4
+#pragma unroll 2
     for (int s = 0; s < n; ++s) {
-      const double v = (double)st[(long long)((slot0 + s) & (kDftSlots - 1)) * np];
+      const long long o = (long long)((slot0 + s) & (kDftSlots - 1)) * np;
+      const double v[kFoldP] = {(double)st0[o], (double)st1[o]};
       const double2* tab = tab0 + (long long)s * nf;
 #pragma unroll
       for (int q = 0; q < kFoldF; ++q) {
         if (decltype(full)::value || q < nfc) {
           const double2 cs = __ldg(&tab[q]);
-          double c = dmul(v, cs.x), d = dmul(v, cs.y);
-          if (decltype(scaled)::value) {
-            c = dmul(c, scale);
-            d = dmul(d, scale);
+#pragma unroll
+          for (int k = 0; k < kFoldP; ++k) {
+            double c = dmul(v[k], cs.x), d = dmul(v[k], cs.y);
+            if (decltype(scaled)::value) {
+              c = dmul(c, scale);
+              d = dmul(d, scale);
+            }
+            re[k][q] = dadd(re[k][q], c);
+            im[k][q] = dsub(im[k][q], d);
           }
-          re[q] = dadd(re[q], c);
-          im[q] = dsub(im[q], d);
         }
       }
     }
@@ -72,12 +84,13 @@ __device__ __forceinline__ void fold_monitor(const MonitorDev& m, const Grid& g,
     if (nfc == kFoldF) window(Yes{}, Yes{}); else window(Yes{}, No{});
   }
 #pragma unroll
-  for (int q = 0; q < kFoldF; ++q) {
-    if (q < nfc) {
-      m.re[(long long)(f0 + q) * np + p] = re[q];
-      m.im[(long long)(f0 + q) * np + p] = im[q];
-    }
-  }
+  for (int c = 0; c < kFoldP; ++c)
+#pragma unroll
+    for (int q = 0; q < kFoldF; ++q)
+      if (q < nfc && (c == 0 || two)) {
+        m.re[(long long)(f0 + q) * np + p[c]] = re[c][q];
+        m.im[(long long)(f0 + q) * np + p[c]] = im[c][q];
+      }
 }
 
 // One grid: blockIdx.z is the monitor.
@@ -98,7 +111,8 @@ __global__ void __launch_bounds__(kFoldThreads) dft_fold_batch(const Args* grids
 }
 
 dim3 fold_grid(long long max_np, int max_nf, int nz) {
-  return dim3((unsigned)((max_np + kFoldThreads - 1) / kFoldThreads),
+  constexpr int per = kFoldThreads * kFoldP;
+  return dim3((unsigned)((max_np + per - 1) / per),
               (unsigned)((max_nf + kFoldF - 1) / kFoldF), (unsigned)nz);
 }
 
