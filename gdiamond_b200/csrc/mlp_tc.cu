@@ -454,11 +454,16 @@ __global__ void __launch_bounds__(FTHREADS, 2) mlp_fused_infer(const __grid_cons
         if (tid == 0) {
           tc_fence_after();
           const uint32_t a0 = smem_u32(act), b0 = smem_u32(sW);
+          // Only the K slices that exist: the activation tile holds no zeros behind a width that
+          // is no multiple of 64, and 0 * (whatever was in shared memory) may be NaN.
+          const int slices = min(TBK / 16, (K - c * TBK + 15) / 16);
 #pragma unroll
-          for (int j = 0; j < TBK / 16; ++j)
+          for (int j = 0; j < TBK / 16; ++j) {
+            if (j >= slices) break;
             umma_bf16(tmem, smem_desc_sbo(a0 + (uint32_t)(c * 8 + 2 * j) * 128u, FACT_K / 8 * 128),
                       smem_desc_sbo(b0 + (uint32_t)j * 256u, TBK / 8 * 128), instr_desc_n(N),
                       (c > 0 || j > 0) ? 1u : 0u);
+          }
           umma_commit(bar);
         }
         ++g;

@@ -204,3 +204,25 @@ def test_fused_training_epoch_equals_separate_launches(dims, members, n, batch):
         net.close()
     assert np.array_equal(out["auto"][0], out["mma_sync"][0])
     assert np.allclose(out["auto"][1], out["mma_sync"][1], rtol=1e-5)
+
+
+# Widths that are no multiple of the 64-wide K chunk: the fused kernel's activation tile is not
+# cleared behind them.  Another network's activations (or NaN) are left in shared memory first.
+@pytest.mark.parametrize("dims", [(6, 96, 32), (6, 160, 96, 64), (5, 32, 224, 32), (64, 96, 96, 96, 32)])
+def test_fused_inference_of_widths_between_chunks(dims):
+    x, _ = data(700, dims, 2)
+    wide = gd.MLP((6, 256, 256, 64), members=2, seed=9)
+    P = wide.get_params()
+    P[:] = np.inf  # its activations become infinite and NaN
+    wide.set_params(P)
+    net = gd.MLP(dims, members=3, seed=4)
+    ref = gd.MLP(dims, members=3, seed=4, gemm="mma_sync")
+    ref.set_params(net.get_params())
+    want = ref.predict(x, members=True)
+    for _ in range(3):
+        wide.predict(data(60000, wide.dims, 1)[0])
+        got = net.predict(x, members=True)
+        for a, b in zip(got, want):
+            assert np.isfinite(a).all() and rel(a, b) <= 1e-3
+    for n in (wide, net, ref):
+        n.close()
