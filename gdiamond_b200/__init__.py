@@ -628,7 +628,8 @@ class MLP:
 
     def set_gemm(self, gemm):
         """GEMM path: "tcgen05" (tensor-memory accumulator), "mma_sync" (warp-level) or "auto"
-        (tcgen05 for products of >= 1024 rows, mma_sync for training minibatches)."""
+        (tcgen05 for products of >= 1024 rows, mma_sync for training minibatches, an epoch
+        in one launch where the network and the minibatch fit)."""
         self._check(self._L.fdtd_mlp_set_gemm(self._h, self.GEMMS[gemm]))
         self.gemm = gemm
 

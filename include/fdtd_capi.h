@@ -354,7 +354,8 @@ typedef struct fdtd_mlp fdtd_mlp;
 
 /* GEMM path of an ensemble: tcgen05.mma with the accumulator in tensor memory, the warp-level
  * mma.sync kernel (the same products), or AUTO (default): tcgen05 for products of >= 1024
- * rows (inference), mma.sync for the short minibatch products of training. */
+ * rows (inference), mma.sync for the short minibatch products of training, whole epochs in one
+ * launch where the network and the minibatch fit (the results of the per-layer launches). */
 typedef enum fdtd_mlp_gemm {
   FDTD_MLP_GEMM_TCGEN05 = 0,
   FDTD_MLP_GEMM_MMA_SYNC = 1,
