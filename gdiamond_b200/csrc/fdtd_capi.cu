@@ -134,7 +134,7 @@ struct fdtd_handle {
   FluxHost flux[kMaxFlux];
   int nflux = 0;
   long long t = 0;
-  int* d_err = nullptr;
+  int* d_err = nullptr;  // error words: of the steps, of the autotuning trials
   fdtd::TiledConfig cfg{0, 0, 0};
   bool cfg_ready = false;
   CUtensorMap maps[2][6];
@@ -378,7 +378,7 @@ fdtd::TiledArgs make_tiled_args(fdtd_handle* h, const fdtd::TiledConfig& c, long
   a.t0 = t0;
   a.dx = h->desc.dx;
   a.zlen = (h->g.nz + c.z_chunks - 1) / c.z_chunks;
-  a.err = h->d_err;
+  a.err = with_io ? h->d_err : h->d_err + 1;  // a trial's outputs are discarded
   for (int k = 0; k < 6; ++k) {
     a.scale[k] = h->scale[k];
     a.inv_scale[k] = h->inv_scale[k];
@@ -451,8 +451,22 @@ std::vector<fdtd::TiledConfig> candidates(const fdtd_handle* h) {
   return out;
 }
 
-// Times every candidate on the current field set (source set -> scratch destination; monitors
-// off, so the simulation state is not changed) and keeps the fastest per step.
+// Reads and clears the error word of the trials.  A trial may take more steps than the caller asked
+// for, so a 16-bit overflow in it says nothing about the run; a copy that never arrived does.
+fdtd_status check_trials(fdtd_handle* h, cudaStream_t st) {
+  int e = 0;
+  CUDA_TRY(h, cudaMemcpyAsync(&e, h->d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(h, cudaMemsetAsync(h->d_err + 1, 0, sizeof(int), st));
+  CUDA_TRY(h, cudaStreamSynchronize(st));
+  if (e & fdtd::kErrTimeout)
+    return fail(h, FDTD_ERR_DEVICE_TIMEOUT,
+                "a device-side bounded wait expired while tuning (error word %d)", e);
+  return FDTD_OK;
+}
+
+// Times candidates on the current field set (source set -> scratch destination; monitors off and
+// errors in a word of their own, so the simulation is not changed): every tile shape at two
+// z-chunk counts, then the other counts of the best shapes.  Keeps the fastest per step.
 fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
   const auto key = std::make_tuple(h->g.nx, h->g.ny, h->g.nz,
                                    (h->cpml_on ? 10000000000LL : 0LL) +
@@ -484,7 +498,7 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
       -> fdtd_status {
     fdtd_status s = ensure_maps(h, c);
     if (s != FDTD_OK) return s;
-    fdtd::TiledArgs a = make_tiled_args(h, c, 0, false);
+    fdtd::TiledArgs a = make_tiled_args(h, c, h->t, false);
     a.S = make_sources(h);  // on a small grid the tile with the source ends last
     CUDA_TRY(h, launch_any(c, a, h->g, st));
     for (int pass = 0; pass < 2; ++pass) {
@@ -510,8 +524,8 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
       spent += warm * 2 * cands[0].blt;
     }
   }
-  // First every tile shape at two z-chunk counts (its largest, and 4), then the other counts of
-  // the eight best shapes.
+  // First every tile shape at its largest z-chunk count and at 4, then the other counts of the eight
+  // best shapes.
   auto shape = [](const fdtd::TiledConfig& c) {
     return std::make_tuple(c.pairs32, c.width, c.rows, c.blt, c.min_blocks);
   };
@@ -559,6 +573,8 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  const fdtd_status s = check_trials(h, st);
+  if (s != FDTD_OK) return s;
   h->cfg = best_c;
   h->cfg_ready = true;
   std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1107,9 +1123,9 @@ fdtd_status fdtd_create(const fdtd_desc* d, fdtd_handle** out) {
                          cudaGetErrorString(e)));
       cudaMemsetAsync(h->F[s][c], 0, bytes, h->stream);
     }
-  if (cudaMalloc(&h->d_err, sizeof(int)) != cudaSuccess)
+  if (cudaMalloc(&h->d_err, 2 * sizeof(int)) != cudaSuccess)
     return bail(fail(h, FDTD_ERR_OOM, "cudaMalloc failed"));
-  cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
+  cudaMemsetAsync(h->d_err, 0, 2 * sizeof(int), h->stream);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess)
     return bail(fail(h, FDTD_ERR_CUDA, "initialisation failed"));
   *out = h;
@@ -2079,6 +2095,8 @@ fdtd_status batch_autotune(fdtd_batch* b, cudaStream_t st) {
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  for (fdtd_handle* h : b->sims)
+    if ((s = check_trials(h, st)) != FDTD_OK) return bfail(b, s, "%s", h->err.c_str());
   b->cfg = best_c;
   b->ctas = best_ctas;
   b->zlen = best_zlen;

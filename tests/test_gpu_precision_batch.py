@@ -351,3 +351,53 @@ def test_16bit_overflow_is_reported_not_silent(storage):
 @pytest.mark.parametrize("blt", [1, 2])
 def test_16bit_20_row_tiles_match_rounded_oracle(storage, blt):
     test_16bit_pairs32_matches_rounded_oracle(storage, blt, 20)
+
+
+def _tuned_and_plain(shape, coefs, sources, t0, fields=None, batch=False):
+    """One step (so one rounding) of an F16 grid that is autotuned and of one with a single
+    configuration."""
+    out = []
+    for kw in (dict(), dict(kernel="tiled_w32p", blt=1, tile_rows=24, z_chunks=1, min_blocks=1)):
+        sim = gd.Simulation(*shape, storage="f16", **kw)
+        sim.set_coefficients(coefs)
+        sim.set_sources(sources)
+        if t0:
+            ck = sim.checkpoint()
+            ck["t"] = t0
+            sim.restore(ck)
+        for c, f in enumerate(fields or []):
+            sim.set_field(c, f)
+        if batch and not kw:
+            b = gd.Batch([sim])
+            b.step(1)
+            b.close()
+        else:
+            sim.step(1)
+        sim.sync()  # raises when a trial marked the run invalid
+        out.append(sim.fields())
+        sim.close()
+    for c in range(6):
+        assert bits_equal(out[0][c], out[1][c]), c
+
+
+@pytest.mark.parametrize("t0,wave", [(0, [0.5, 1e9, 1e9, 1e9, 1e9, 1e9]),
+                                     (10, [1e9] * 10 + [0.5, 1e9, 1e9])])
+def test_autotuning_trials_do_not_mark_the_run_invalid(t0, wave):
+    """A source that overflows FP16 storage in steps which the run does not take (later ones than
+    asked for, or those before the step it resumes at) but an autotuning trial might."""
+    shape = (70, 41, 23 + t0)  # a shape of its own: tuned configurations are kept per shape
+    src = [dict(component="Jz", wave=np.asarray(wave, np.float32), i=35, j=20, k=11)]
+    _tuned_and_plain(shape, W.vacuum_coefficients(shape), src, t0)
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_autotuning_trials_of_growing_fields_do_not_mark_the_run_invalid(batch):
+    """A medium with gain (E grows 16-fold a step): one step stays in FP16's range, a trial of
+    two or more does not."""
+    shape = (72 + batch, 41, 23)
+    coefs = [c.copy() for c in W.vacuum_coefficients(shape)]
+    for c in range(3):
+        coefs[c] = np.full_like(coefs[c], 16.0)
+    n = shape[0] * shape[1] * shape[2]
+    f = np.random.default_rng(3).uniform(500, 1000, n).astype(np.float32)
+    _tuned_and_plain(shape, coefs, [], 0, [f] * 3, batch)
