@@ -6,10 +6,69 @@
 //   2-byte elements.  Pad columns i >= Nx are zero and never written.
 #pragma once
 
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <utility>
+
 namespace fdtd {
+
+// The id of the current context, unique in the process's life; 0 when there is none.
+inline unsigned long long context_id() {
+  static const PFN_cuCtxGetId_v12000 fn = [] {
+    void* q = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &q, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess)
+      q = nullptr;
+    return reinterpret_cast<PFN_cuCtxGetId_v12000>(q);
+  }();
+  unsigned long long id = 0;
+  return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// Contexts (one a device) in which a kernel's attributes have been set.
+constexpr int kAttrDevices = 16;
+struct AttributesSet {
+  std::atomic<unsigned long long> context[kAttrDevices] = {};
+};
+
+// Launches a kernel that needs function attributes (such as more dynamic shared memory than the
+// default).  `set` sets them for the current device, which costs as much as a small launch, so only
+// before the first launch in a context: cudaDeviceReset ends the context and drops them.
+template <typename Set, typename... P, typename... A>
+cudaError_t launch_with(AttributesSet& done, Set set, void (*kernel)(P...), dim3 grid, dim3 block,
+                        size_t smem, cudaStream_t st, A&&... args) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long id = dev < kAttrDevices ? context_id() : 0;
+  if (id == 0 || done.context[dev].load(std::memory_order_relaxed) != id) {
+    if ((e = set()) != cudaSuccess) return e;
+    if (id != 0) done.context[dev].store(id);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  const cudaError_t last = cudaGetLastError();
+  return e != cudaSuccess ? e : last;
+}
+
+// The same for a kernel that only needs its dynamic shared memory.
+template <typename... P, typename... A>
+cudaError_t launch_smem(AttributesSet& done, void (*kernel)(P...), dim3 grid, dim3 block,
+                        size_t smem, cudaStream_t st, A&&... args) {
+  auto set = [&] {
+    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  };
+  return launch_with(done, set, kernel, grid, block, smem, st, std::forward<A>(args)...);
+}
 
 constexpr int kMaxSources = 8;
 constexpr int kMaxMonitors = 12;  // a flux monitor takes six

@@ -2,26 +2,9 @@
 #pragma once
 
 #include <cuda.h>  // CUtensorMap (types only; the driver entry point is fetched at run time)
-
-#include <atomic>
-
 #include "fdtd_common.cuh"
 
 namespace fdtd {
-
-// Opts a kernel in to `bytes` of dynamic shared memory once per device (`done`: a bit per device
-// ordinal, one word per kernel instance): the call costs as much as a small launch.
-inline cudaError_t allow_smem(const void* kernel, size_t bytes,
-                              std::atomic<unsigned long long>& done) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (bit && (done.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done.fetch_or(bit);
-  return e;
-}
 
 struct FieldPtrs {
   float* f[6];  // Ex Ey Ez Hx Hy Hz, pitched

@@ -303,11 +303,8 @@ __global__ void __launch_bounds__(32 * TY) fdtd_tiled(const __grid_constant__ Ti
 template <int B, int TY>
 cudaError_t launch_one(const TiledArgs& a, dim3 grid, cudaStream_t st) {
   using K = Tiled<B, TY>;
-  static std::atomic<unsigned long long> done{0};
-  cudaError_t e = allow_smem(reinterpret_cast<const void*>(&fdtd_tiled<B, TY>), K::SMEM, done);
-  if (e != cudaSuccess) return e;
-  fdtd_tiled<B, TY><<<grid, dim3(32, TY), K::SMEM, st>>>(a);
-  return cudaGetLastError();
+  static AttributesSet done;
+  return launch_smem(done, fdtd_tiled<B, TY>, grid, dim3(32, TY), K::SMEM, st, a);
 }
 
 template <int TY>

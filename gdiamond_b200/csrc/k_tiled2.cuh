@@ -722,23 +722,17 @@ __global__ void __launch_bounds__(TY * W / 2, (batch_min_blocks<TY, W>()))
 template <typename S, int B, int TY, int MINB, int W = 64, typename SH = S>
 cudaError_t launch_one2(const TiledArgs& a, dim3 grid, cudaStream_t st) {
   using K = Tiled2<S, B, TY, W, SH>;
-  static std::atomic<unsigned long long> done{0};
-  cudaError_t e = allow_smem(reinterpret_cast<const void*>(&fdtd_tiled2<S, B, TY, MINB, W, SH>),
-                             K::SMEM, done);
-  if (e != cudaSuccess) return e;
-  fdtd_tiled2<S, B, TY, MINB, W, SH><<<grid, dim3(32, K::THREADS / 32), K::SMEM, st>>>(a);
-  return cudaGetLastError();
+  static AttributesSet done;
+  return launch_smem(done, fdtd_tiled2<S, B, TY, MINB, W, SH>, grid, dim3(32, K::THREADS / 32),
+                     K::SMEM, st, a);
 }
 
 template <typename S, int B, int TY, int W = 64, typename SH = S>
 cudaError_t launch_batch_one(const BatchArgs& b, int ctas, cudaStream_t st) {
   using K = Tiled2<S, B, TY, W, SH>;
-  static std::atomic<unsigned long long> done{0};
-  cudaError_t e = allow_smem(reinterpret_cast<const void*>(&fdtd_tiled2_batch<S, B, TY, W, SH>),
-                             K::SMEM, done);
-  if (e != cudaSuccess) return e;
-  fdtd_tiled2_batch<S, B, TY, W, SH><<<ctas, dim3(32, K::THREADS / 32), K::SMEM, st>>>(b);
-  return cudaGetLastError();
+  static AttributesSet done;
+  return launch_smem(done, fdtd_tiled2_batch<S, B, TY, W, SH>, dim3(ctas),
+                     dim3(32, K::THREADS / 32), K::SMEM, st, b);
 }
 
 // 32-wide rows (two per warp): 20 and 24 rows (10 and 12 warps, BLT 1-2, registers capped for two

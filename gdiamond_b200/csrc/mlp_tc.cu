@@ -19,7 +19,6 @@
 // (decided block-wide with __syncthreads_or), waits (bounded) for what it issued, skips the
 // epilogue, frees its TMEM and returns.
 #include <algorithm>
-#include <atomic>
 
 #include "fdtd_common.cuh"
 #include "mlp.cuh"
@@ -289,20 +288,10 @@ __global__ void __launch_bounds__(128) gemm_tc(int M, int N, int K, Operand A, O
 template <bool TA, bool TB, int EPI, int BN>
 cudaError_t launch_bn(int M, int N, int K, const Operand& A, const Operand& B, const Epilogue& ep,
                       int members, cudaStream_t st, int* err) {
-  static std::atomic<unsigned long long> set_on{0};  // devices (bit per ordinal < 64) done
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (!(set_on.load() & bit) || !bit) {
-    e = cudaFuncSetAttribute(gemm_tc<TA, TB, EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)TcSmem<BN>::BYTES);
-    if (e != cudaSuccess) return e;
-    set_on.fetch_or(bit);
-  }
+  static AttributesSet done;
   const dim3 grid((N + BN - 1) / BN, (M + TBM - 1) / TBM, members);
-  gemm_tc<TA, TB, EPI, BN><<<grid, 128, TcSmem<BN>::BYTES, st>>>(M, N, K, A, B, ep, err);
-  return cudaGetLastError();
+  return launch_smem(done, gemm_tc<TA, TB, EPI, BN>, grid, dim3(128), TcSmem<BN>::BYTES, st, M, N,
+                     K, A, B, ep, err);
 }
 
 // ------------------------------------------------------------------- fused ensemble inference
@@ -576,24 +565,15 @@ bool mlp_fused_supported(const int* dims, int L) {
 }
 
 cudaError_t launch_mlp_fused(const FusedArgs& a, int members, cudaStream_t st) {
-  static std::atomic<unsigned long long> set_on{0};
-  int dev = 0;
+  static AttributesSet done;
+  int dev = 0, nsm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (!(set_on.load() & bit) || !bit) {
-    e = cudaFuncSetAttribute(mlp_fused_infer, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)F_SMEM);
-    if (e != cudaSuccess) return e;
-    set_on.fetch_or(bit);
-  }
-  int nsm = 0;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   const long long nblk = (a.n + FROWS - 1) / FROWS, ntiles = nblk * members;
   if (ntiles > 0x7fffffffLL - 2 * nsm) return cudaErrorInvalidValue;
-  mlp_fused_infer<<<(unsigned)std::min<long long>(ntiles, 2 * nsm), FTHREADS, F_SMEM, st>>>(
-      a, (int)nblk, (int)ntiles);
-  return cudaGetLastError();
+  return launch_smem(done, mlp_fused_infer, dim3((unsigned)std::min<long long>(ntiles, 2 * nsm)),
+                     dim3(FTHREADS), F_SMEM, st, a, (int)nblk, (int)ntiles);
 }
 
 }  // namespace mlp

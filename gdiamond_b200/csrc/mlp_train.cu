@@ -22,8 +22,6 @@
 // FP32 accumulators over k in steps of 16, the same epilogues, column sums in row order, the same
 // Adam update.  A tcgen05 tile has 128 rows; a minibatch of 64 would leave half of it empty and
 // the products are bound by latency, not by tensor throughput.
-#include <atomic>
-
 #include "fdtd_common.cuh"
 #include "mlp.cuh"
 
@@ -408,21 +406,28 @@ bool train_epoch_supported(const int* dims, int L, int batch) {
 
 namespace {
 
-// Sets the kernel up on the current device, once; *ok: the device can hold a cluster of CTAS.
 template <int CTAS>
-cudaError_t set_up(bool* ok) {
+cudaError_t set_attributes() {
+  cudaError_t e = cudaFuncSetAttribute(
+      train_epoch<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  if (e == cudaSuccess && CTAS > 8)
+    e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+
+// Whether the current device can hold a cluster of CTAS; asked once.
+template <int CTAS>
+cudaError_t cluster_fits(bool* ok) {
   static std::atomic<unsigned long long> done{0}, fits{0};  // a bit per device ordinal < 64
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  *ok = (fits.load() & bit) != 0;
-  if (bit && (done.load() & bit)) return cudaSuccess;
-  e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kSmem);
-  if (e == cudaSuccess && CTAS > 8)
-    e = cudaFuncSetAttribute(train_epoch<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return e;
+  if (done.load() & bit) {
+    *ok = (fits.load() & bit) != 0;
+    return cudaSuccess;
+  }
+  if ((e = set_attributes<CTAS>()) != cudaSuccess) return e;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = CTAS;
@@ -444,23 +449,24 @@ cudaError_t set_up(bool* ok) {
   return cudaSuccess;
 }
 
+template <int CTAS>
+cudaError_t launch(const TrainArgs& a, int members, cudaStream_t st) {
+  static AttributesSet done;
+  return launch_with(done, set_attributes<CTAS>, train_epoch<CTAS>, dim3(CTAS * members),
+                     dim3(kThreads), kSmem, st, a);
+}
+
 }  // namespace
 
 // A member's cluster: 16 CTAs (more than the portable 8) for small ensembles, whose members then
 // all run at once, where the device has a GPC with 16 free SMs; 8 otherwise.
 cudaError_t launch_train_epoch(const TrainArgs& a, int members, cudaStream_t st) {
   bool ok = false;
-  cudaError_t e;
   if (members <= 4) {
-    if ((e = set_up<16>(&ok)) != cudaSuccess) return e;
-    if (ok) {
-      train_epoch<16><<<16 * members, kThreads, kSmem, st>>>(a);
-      return cudaGetLastError();
-    }
+    const cudaError_t e = cluster_fits<16>(&ok);
+    if (e != cudaSuccess) return e;
   }
-  if ((e = set_up<8>(&ok)) != cudaSuccess) return e;
-  train_epoch<8><<<8 * members, kThreads, kSmem, st>>>(a);
-  return cudaGetLastError();
+  return ok ? launch<16>(a, members, st) : launch<8>(a, members, st);
 }
 
 }  // namespace mlp

@@ -50,3 +50,55 @@ def test_expired_wait_reports_timeout_and_handle_recovers(family, blt, rows, sto
     else:
         assert all(np.isfinite(f).all() for f in sim.fields())
     sim.close()
+
+
+_RESET = """
+import ctypes, sys
+import numpy as np
+import gdiamond_b200 as gd
+from gdiamond_b200 import workloads as W
+
+def work():
+    out = []
+    shape = (70, 52, 41)
+    for kernel, rows in (("tiled_w32", 16), ("tiled_w64", 16), ("tiled_w32p", 32)):
+        sim = gd.Simulation(*shape, kernel=kernel, blt=2, tile_rows=rows, z_chunks=2, min_blocks=1)
+        sim.set_coefficients(W.vacuum_coefficients(shape))
+        sim.set_sources([dict(component="Jz", wave=W.gaussian_wave(8, delay=3.0), i=35, j=26, k=20)])
+        if kernel == "tiled_w32p":
+            b = gd.Batch([sim])
+            b.step(5)  # the last step's instance is first launched while the graph is captured
+            b.close()
+        sim.step(4)
+        sim.sync()
+        out += sim.fields()
+        sim.close()
+    rng = np.random.default_rng(0)
+    x, y = rng.normal(size=(2048, 6)).astype(np.float32), rng.normal(size=(2048, 32)).astype(np.float32)
+    for members in (2, 5):
+        net = gd.MLP((6, 64, 32), members=members, seed=1)
+        net.set_data(x, y)
+        net.train(1, batch=64)
+        out += [net.get_params()] + list(net.predict(x)) + [net.grad(x, y)[1]]
+        net.close()
+    return out
+
+first = work()
+rt = ctypes.CDLL([l.split()[-1] for l in open("/proc/self/maps") if "libcudart.so" in l][0])
+assert rt.cudaDeviceSynchronize() == 0 and rt.cudaDeviceReset() == 0
+for a, b in zip(first, work()):
+    assert np.array_equal(a, b) or np.allclose(a, b, rtol=1e-4, atol=1e-6)
+print("same after the reset")
+"""
+
+
+def test_new_handles_work_after_a_device_reset():
+    """cudaDeviceReset ends the process's context and with it every kernel attribute that was
+    set; handles made afterwards run as the first ones did."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _RESET], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "same after the reset" in r.stdout, r.stderr[-2000:]
