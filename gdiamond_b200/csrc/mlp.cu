@@ -293,7 +293,8 @@ struct fdtd_mlp {
   __nv_bfloat16* gbf[2] = {nullptr, nullptr};  // their BF16 copies
   float* tgt = nullptr;                        // [E][cap][out]
   float* xin = nullptr;                        // FP32 input staging [cap][in]
-  std::vector<__nv_bfloat16*> gl;  // train_epoch: gl[l] [E][cap][dims[l+1]], gradients of layer l
+  // train_epoch: gl[l] [E][kTrainMaxRows][dims[l+1]], gradients of layer l
+  std::vector<__nv_bfloat16*> gl;
   float* pred = nullptr;  // fused inference: every member's outputs of a chunk of rows
   size_t pred_cap = 0;
   // training workspace, kept between calls: row order [E][n], summed losses, bias corrections
@@ -331,8 +332,6 @@ void free_workspace(fdtd_mlp* m) {
     m->g[i] = nullptr;
     m->gbf[i] = nullptr;
   }
-  for (auto p : m->gl) cudaFree(p);
-  m->gl.clear();
   cudaFree(m->tgt);
   cudaFree(m->xin);
   m->tgt = nullptr;
@@ -372,6 +371,24 @@ cudaError_t grow(fdtd_mlp* m, T** p, size_t* cap, size_t count) {
   *cap = 0;
   if ((e = cudaMalloc(p, count * sizeof(T))) == cudaSuccess) *cap = count;
   return e;
+}
+
+// The workspace of one-launch epochs of `steps` minibatches; false when there is no room for it.
+bool epoch_workspace(fdtd_mlp* m, int steps) {
+  if (m->gl.empty()) {
+    m->gl.assign(m->L, nullptr);
+    for (int l = 0; l < m->L; ++l)
+      if (cudaMalloc(&m->gl[l], (size_t)m->E * fdtd::mlp::kTrainMaxRows * m->dims[l + 1] *
+                                    sizeof(__nv_bfloat16)) != cudaSuccess) {
+        for (auto p : m->gl) cudaFree(p);
+        m->gl.clear();
+        cudaGetLastError();
+        return false;
+      }
+  }
+  if (grow(m, &m->corr, &m->corr_cap, (size_t)steps) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -497,6 +514,7 @@ void destroy(fdtd_mlp* m) {
   cudaFree(m->perm);
   cudaFree(m->dloss);
   cudaFree(m->corr);
+  for (auto p : m->gl) cudaFree(p);
   cudaFree(m->X);
   cudaFree(m->Y);
   if (m->st) cudaStreamDestroy(m->st);
@@ -741,25 +759,17 @@ fdtd_status fdtd_mlp_train(fdtd_mlp* m, int32_t epochs, int32_t batch, float lr,
     return make_float2((float)(1.0 - std::pow((double)b1, (double)m->adam_t)),
                        (float)(1.0 - std::pow((double)b2, (double)m->adam_t)));
   };
-  // AUTO: the whole epoch in one launch where the network and the batch fit it (mlp_train.cu).
+  // AUTO: the whole epoch in one launch where the network and the batch fit it (mlp_train.cu) and
+  // there is room for its workspace; the same results a launch per product at a time otherwise.
+  const int steps = (int)((n + mb - 1) / mb);
   const bool fused = m->gemm_kind == FDTD_MLP_GEMM_AUTO &&
-                     fdtd::mlp::train_epoch_supported(m->dims.data(), m->L, mb);
+                     fdtd::mlp::train_epoch_supported(m->dims.data(), m->L, mb) &&
+                     epoch_workspace(m, steps);
   fdtd::mlp::TrainArgs ta{};
   std::vector<float2> hc;
   if (fused) {
-    if (m->gl.empty()) {
-      m->gl.assign(m->L, nullptr);
-      for (int l = 0; l < m->L; ++l)
-        if (cudaMalloc(&m->gl[l], m->E * m->cap * m->dims[l + 1] * sizeof(__nv_bfloat16)) !=
-            cudaSuccess) {
-          for (auto p : m->gl) cudaFree(p);
-          m->gl.clear();
-          cudaGetLastError();
-          return mfail(m, FDTD_ERR_CUDA, "training workspace allocation failed");
-        }
-    }
     ta.L = m->L;
-    ta.steps = (int)((n + mb - 1) / mb);
+    ta.steps = steps;
     ta.batch = mb;
     for (int l = 0; l <= m->L; ++l) {
       ta.dims[l] = m->dims[l];
@@ -785,7 +795,6 @@ fdtd_status fdtd_mlp_train(fdtd_mlp* m, int32_t epochs, int32_t batch, float lr,
     ta.b1 = b1;
     ta.b2 = b2;
     ta.eps = eps;
-    MCUDA(m, grow(m, &m->corr, &m->corr_cap, (size_t)ta.steps));
     ta.corr = m->corr;
     hc.resize(ta.steps);
   }

@@ -93,7 +93,7 @@ struct TrainArgs {
   __nv_bfloat16* wbf;                           // [members][P]
   __nv_bfloat16* act[kFusedMaxLayers + 1];      // [members][cap][dims[l]], l >= 1
   float* z[kFusedMaxLayers];                    // [members][cap][dims[l+1]]
-  __nv_bfloat16* gbf[kFusedMaxLayers];          // [members][cap][dims[l+1]]
+  __nv_bfloat16* gbf[kFusedMaxLayers];          // [members][kTrainMaxRows][dims[l+1]]
   float* loss;                     // [members]: summed squared errors are added
   const float2* corr;              // [steps]: Adam's bias corrections
   float lr, b1, b2, eps;

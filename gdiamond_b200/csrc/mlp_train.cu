@@ -241,7 +241,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
               const float d0 = v0 - yv[j][h].x, d1 = v1 - yv[j][h].y;
               loss += d0 * d0 + d1 * d1;
               const float g0 = scale * d0, g1 = scale * d1;
-              *reinterpret_cast<__nv_bfloat162*>(a.gbf[l] + o) =
+              *reinterpret_cast<__nv_bfloat162*>(a.gbf[l] + ((long long)e * kRows + r) * N + col) =
                   __halves2bfloat162(__float2bfloat16_rn(g0), __float2bfloat16_rn(g1));
               sG[r * 33 + lc] = g0;
               sG[r * 33 + lc + 1] = g1;
@@ -274,7 +274,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
         gather_rows(sB, a.X, sRow, in0, M, M16, in_pad);
       }
       if (l == L - 1) cluster_wait();  // below, the wait for dX_l is also the next layer's
-      copy_rows(sA, LD, a.gbf[l] + (long long)e * a.cap * o, o, M, M16, o);
+      copy_rows(sA, LD, a.gbf[l] + (long long)e * kRows * o, o, M, M16, o);
       cp_wait();
       __syncthreads();
       if (l > 0) {  // G_{l-1} = (G_l W_l) * GELU'(z_{l-1})
@@ -299,7 +299,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kThreads, 1)
             for (int h = 0; h < 2; ++h) {
               const int r = m0 + gid + 8 * h, lc = n0 + 8 * j + 2 * tig;
               if (r >= M) continue;
-              const long long q = ((long long)e * a.cap + r) * in + cfirst + lc;
+              const long long q = ((long long)e * kRows + r) * in + cfirst + lc;
               const float g0 = acc[j][2 * h] * gelu_grad(zv[j][h].x);
               const float g1 = acc[j][2 * h + 1] * gelu_grad(zv[j][h].y);
               *reinterpret_cast<__nv_bfloat162*>(a.gbf[l - 1] + q) =

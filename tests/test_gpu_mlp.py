@@ -226,3 +226,55 @@ def test_fused_inference_of_widths_between_chunks(dims):
             assert np.isfinite(a).all() and rel(a, b) <= 1e-3
     for n in (wide, net, ref):
         n.close()
+
+
+def test_training_workspace_does_not_grow_with_an_earlier_prediction():
+    """The one-launch epoch holds gradients of at most 128 rows a member, whatever number of rows
+    an earlier call of the layer-by-layer path sized its own workspace for."""
+    import torch
+    dims, members = (6, 144, 144, 48), 16
+    x, y = data(65536, dims, 1)
+    net = gd.MLP(dims, members=members, seed=2)
+    net.predict(x)  # widths that are no multiples of 32: a layer at a time
+    net.set_data(x[:500], y[:500])
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    net.train(1, batch=64)
+    used = before - torch.cuda.mem_get_info()[0]
+    net.close()
+    # gradients: 16 members x 128 rows x 336 columns x 2 bytes = 1.4 MB; allocations of 2 MB each
+    assert used <= 32 << 20, used
+
+
+def test_training_without_room_for_the_epoch_workspace():
+    """When the one-launch epoch's gradients cannot be allocated, the separate launches, which need
+    no more memory than they hold, train the same parameters."""
+    import ctypes
+    import torch
+    dims, members = (6, 256, 256, 256, 64), 64  # gradients: 4 MB a hidden layer
+    x, y = data(200, dims, 3)
+    want = gd.MLP(dims, members=members, seed=6, gemm="mma_sync")
+    net = gd.MLP(dims, members=members, seed=6, gemm="mma_sync")
+    for m in (want, net):
+        m.set_data(x, y)
+        m.train(1, batch=128, lr=1e-3, seed=3)
+    net.set_gemm("auto")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    rt = ctypes.CDLL([q.split()[-1] for q in open("/proc/self/maps") if "libcudart.so" in q][0])
+    hold = []
+    for size in (1 << 30, 1 << 26, 1 << 21):  # allocations are made of 2 MB pages
+        p = ctypes.c_void_p()
+        while rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0:
+            hold.append(p)
+            p = ctypes.c_void_p()
+        rt.cudaGetLastError()
+    try:
+        net.train(1, batch=128, lr=1e-3, seed=4)
+    finally:
+        for p in hold:
+            rt.cudaFree(p)
+    want.train(1, batch=128, lr=1e-3, seed=4)
+    assert np.array_equal(net.get_params(), want.get_params())
+    want.close()
+    net.close()
