@@ -349,3 +349,61 @@ def test_cpml_odd_rows_and_partial_faces_match_oracle(shape, L, faces):
     b.close()
     for s in sims:
         s.close()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_cpml_batch_of_more_grids_than_a_launch_holds(use_graph):
+    """35 uneven grids (two launches a half step) equal the same grids stepped alone."""
+    rng = np.random.default_rng(8)
+    shapes = [tuple(int(v) for v in rng.integers(12, 29, 3)) for _ in range(35)]
+    freqs = W.source_band(3, period=9.0, width=6.0)
+    pairs = []
+    for n, shape in enumerate(shapes):
+        pairs.append([_cpml_sim(shape, n % 5, L=4, flux_k=shape[2] - 6, freqs=freqs)
+                      for _ in range(2)])
+    b = gd.Batch([p[0][0] for p in pairs])
+    for T in (19, 2):
+        b.step(T, use_graph=use_graph)
+        for (s, m), (r, rm) in pairs:
+            r.step(T)
+            s.sync()
+            assert_fields_match(s.fields(), r.fields(), f"grid {s.shape}")
+            for got, want in zip(_read(s, m), _read(r, rm)):
+                assert np.array_equal(got, want)
+    b.close()
+    for p in pairs:
+        for s, _ in p:
+            s.close()
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_cpml_dft_sums_across_ring_wraps_match_host_sums(batch):
+    """290 steps (more than two staging rings of 128) in calls of 200 and 90, so a ring is folded
+    inside a call and at its end and wraps at an odd slot: DFT sums against FP64 host sums of the
+    plane read after every step (rel. 1e-12: the tables' cosines are the C library's)."""
+    shape, L, nf = (22, 19, 18), 4, 5
+    nx, ny, nz = shape
+    coefs = W.vacuum_coefficients(shape)
+    w = W.gaussian_wave(300, delay=20.0, width=6.0, period=6.0)
+    src = [dict(component="Jz", wave=w, i=nx // 2, j=ny // 2, k=nz // 2)]
+    freqs = W.source_band(nf, period=6.0, width=3.0)
+    sim = make(shape, coefs, src, L)
+    mid = sim.add_dft_monitor("Ez", nz // 2, freqs)
+    b = gd.Batch([sim]) if batch else sim
+    b.step(200)
+    b.step(90)
+    sim.sync()
+    got = np.stack(sim.get_dft(mid))
+    one = make(shape, coefs, src, L)
+    want = np.zeros((2, nf, ny, nx))
+    for t in range(290):
+        one.step(1)
+        v = one.get_field("Ez").reshape(nz, ny, nx)[nz // 2].astype(np.float64)
+        ph = 2 * np.pi * freqs * (t * DT)
+        want[0] += v * np.cos(ph)[:, None, None]
+        want[1] -= v * np.sin(ph)[:, None, None]
+    assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+    if batch:
+        b.close()
+    one.close()
+    sim.close()

@@ -278,3 +278,18 @@ def test_training_without_room_for_the_epoch_workspace():
     assert np.array_equal(net.get_params(), want.get_params())
     want.close()
     net.close()
+
+
+def test_fused_inference_over_more_rows_than_a_chunk():
+    """262144 rows and 129 more (the second chunk's offsets and short copies), then a few rows in
+    the same workspace, against the layer-by-layer path."""
+    dims = (6, 32, 32)
+    nets = [gd.MLP(dims, members=2, seed=3, gemm=g) for g in ("auto", "mma_sync")]
+    for n in (262144 + 129, 200):
+        x, _ = data(n, dims, n & 15)
+        got, want = (net.predict(x, members=True) for net in nets)
+        for a, b in zip(got, want):
+            assert a.shape == b.shape and rel(a, b) <= 1e-3
+            assert rel(a[..., -129:, :], b[..., -129:, :]) <= 1e-3
+    for net in nets:
+        net.close()
