@@ -407,3 +407,25 @@ def test_cpml_dft_sums_across_ring_wraps_match_host_sums(batch):
         b.close()
     one.close()
     sim.close()
+
+
+# Marches of one, two, four and eight planes (the fewest that give every SM its blocks), the last
+# chunk short.
+@pytest.mark.parametrize("shape", [(33, 29, 19), (97, 95, 71), (129, 127, 75), (190, 230, 67)])
+def test_cpml_chunk_lengths_match_oracle(shape):
+    L, T = 6, 5
+    nx, ny, nz = shape
+    eps = np.random.default_rng(6).choice([1.0, 1.0, 2.5], nx * ny * nz).astype(np.float32)
+    coefs = W.reference_coefficients(shape, eps_re=eps, t_pml=0)
+    w = W.gaussian_wave(T, delay=2.0, width=2.0, period=4.0)
+    src = [dict(component="Jz", wave=w, i=nx // 2, j=ny // 2, k=k) for k in (3, nz // 2, nz - 4)]
+    src.append(dict(component="Mx", wave=w, k=nz // 2, kind=gd.SRC_PLANE_Z))
+    sim = make(shape, coefs, src, L)
+    f = [np.random.default_rng(c).normal(size=nx * ny * nz).astype(np.float32) for c in range(6)]
+    for c in range(6):
+        sim.set_field(c, f[c])
+    sim.step(T)
+    F_ref = cpml.run(shape, coefs, T, sim.cpml_tables(), sources=[osrc(s) for s in src], dx=DX,
+                     fields=f)
+    assert_fields_match(sim.fields(), F_ref, f"cpml {shape}")
+    sim.close()
