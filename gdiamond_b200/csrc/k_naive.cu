@@ -224,9 +224,13 @@ void naive_step_t(const Grid& g, const FieldPtrs& F, const CoefArrays& A, const 
                   cudaStream_t st, int* launches) {
   const long long pairs = (long long)((g.nx + 1) / 2) * g.ny;
   const long long nb = (pairs + kNaiveThreads - 1) / kNaiveThreads;
-  // planes per march: at least 8 blocks per SM before it gets longer
+  // planes per march: at least 8 blocks per SM before it gets longer, and single planes where pairs of
+  // them leave fewer than 4 (a march is then only a chain of loads: FP64 48^3 8.1 us a step with one
+  // plane, 11.3 with two; 80^3 14.3 and 12.3)
+  const auto blocks = [&](int planes) { return nb * ((g.nz + planes - 1) / planes); };
   int zc = 16;
-  while (zc > 2 && nb * ((g.nz + zc - 1) / zc) < 148 * 8) zc /= 2;
+  while (zc > 2 && blocks(zc) < 148 * 8) zc /= 2;
+  if (blocks(zc) < 148 * 4) zc = 1;
   zc = std::max(zc, (g.nz + 65534) / 65535);
   const dim3 grd((unsigned)nb, (unsigned)((g.nz + zc - 1) / zc));
   if (mat) {

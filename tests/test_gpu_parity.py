@@ -396,3 +396,26 @@ def test_checkpoint_resume_continues_bit_for_bit(storage):
     assert all(np.array_equal(x, y) for x, y in zip(got["dft"][0], want["dft"][0]))
     a.close()
     c.close()
+
+
+# Marches of the naive kernel of one plane, two and four, the last chunk short.
+@pytest.mark.parametrize("shape", [(45, 33, 21), (63, 64, 81), (129, 127, 75)])
+@pytest.mark.parametrize("percell", [False, True])
+def test_naive_chunk_lengths_match_oracle(shape, percell):
+    T, n = 5, shape[0] * shape[1] * shape[2]
+    rng = np.random.default_rng(12)
+    eps = rng.uniform(1.0, 12.0, n) if percell else rng.choice([1.0, 2.5], n)
+    coefs = W.reference_coefficients(shape, eps_re=eps.astype(np.float32), t_pml=6)
+    w = W.gaussian_wave(T, delay=2.0, width=2.0, period=4.0)
+    src = [dict(component="Jz", wave=w, i=shape[0] // 2, j=shape[1] // 2, k=k)
+           for k in (1, shape[2] // 2, shape[2] - 2)]
+    f = [rng.normal(size=n).astype(np.float32) for _ in range(6)]
+    sim = gd.Simulation(*shape, kernel="naive")
+    sim.set_coefficients(coefs)
+    sim.set_sources(src)
+    for c in range(6):
+        sim.set_field(c, f[c])
+    sim.step(T)
+    assert_fields_match(sim.fields(), oracle.run(shape, coefs, T, sources=[osrc(s) for s in src],
+                                                 fields=f), f"naive {shape}")
+    sim.close()
