@@ -7,9 +7,10 @@
 // of distinct tuples.  This file builds that map on the device:
 //   1. insert: hash each cell's 12 words (bitwise) into an open-addressing table of 2^20
 //      64-bit keys; a key's representative is its first cell (lowest index);
-//   2. assign: number the keys in the order of their representatives and copy each one's tuple
-//      into the table.  Neighbouring cells of a graded layer then have neighbouring table
-//      entries, and a warp's coefficient loads touch a few cache lines instead of one per cell;
+//   2. assign: number the keys in the order of their representatives (bucketed by ranges of cells,
+//      then counted within the bucket) and copy each one's tuple into the table.  Neighbouring
+//      cells of a graded layer then have neighbouring table entries, and a warp's coefficient
+//      loads touch a few cache lines instead of one per cell;
 //   3. map: write each cell's id and compare its 12 words with the table entry, so a 64-bit
 //      hash collision is detected (the map is then rejected) instead of silently merged; count
 //      the cells of each id and report the id held by the most cells (the kernels' fast path
@@ -27,6 +28,7 @@ constexpr uint32_t kSlots = 1u << kSlotBits;
 constexpr unsigned long long kEmpty = ~0ull;
 constexpr int kMaxProbe = 4096;
 constexpr int kMaxMaterials = 65536;
+constexpr int kBuckets = 4096;  // of representatives, by ranges of cells
 
 struct Scratch {
   unsigned long long keys[kSlots];
@@ -39,6 +41,9 @@ struct Scratch {
   unsigned int count[kMaxMaterials];  // cells per id
   uint32_t slot[kMaxMaterials];            // occupied slots, in no order
   unsigned long long first[kMaxMaterials]; // their representatives
+  unsigned long long sorted[kMaxMaterials];  // the representatives by bucket
+  uint32_t start[kBuckets + 1];              // first entry of a bucket (before: their counts)
+  uint32_t cursor[kBuckets];
 };
 
 struct Coef12 {
@@ -75,6 +80,7 @@ __global__ void k_reset(Scratch* s) {
     s->ids[q] = 0xFFFFFFFFu;
   }
   if (q < (uint32_t)kMaxMaterials) s->count[q] = 0;
+  if (q <= (uint32_t)kBuckets) s->start[q] = 0;
   if (q == 0) s->nuniq = s->nid = s->flags = s->mode = 0;
 }
 
@@ -106,31 +112,60 @@ __global__ void k_insert(Grid g, Coef12 C, Scratch* s, long long n) {
   }
 }
 
-// Lists the occupied slots and their representatives.
-__global__ void k_list(Scratch* s) {
+// Lists the occupied slots and their representatives and counts these in buckets of 2^shift cells.
+__global__ void k_list(Scratch* s, int shift) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= kSlots || s->keys[q] == kEmpty) return;
   const unsigned int n = atomicAdd(&s->nid, 1u);
   if (n >= (unsigned)kMaxMaterials) return;  // rejected on the host
   s->slot[n] = q;
   s->first[n] = s->rep[q];
+  atomicAdd(&s->start[s->rep[q] >> shift], 1u);
 }
 
-// Entry n of the list gets the id that counts the representatives before its own.
-__global__ void __launch_bounds__(256) k_assign(Coef12 C, Scratch* s, Material* table, int nuniq) {
-  __shared__ unsigned long long tile[256];
-  const int n = blockIdx.x * 256 + threadIdx.x;
-  const unsigned long long r = n < nuniq ? s->first[n] : 0;
-  int id = 0;
-  for (int t0 = 0; t0 < nuniq; t0 += 256) {
+// Counts to first entries; one block of 1024 threads.
+__global__ void __launch_bounds__(1024) k_scan(Scratch* s) {
+  constexpr int P = kBuckets / 1024;
+  __shared__ uint32_t sum[1024];
+  const int t = threadIdx.x;
+  uint32_t c[P], mine = 0;
+#pragma unroll
+  for (int q = 0; q < P; ++q) mine += c[q] = s->start[t * P + q];
+  sum[t] = mine;
+  for (int d = 1; d < 1024; d *= 2) {
     __syncthreads();
-    if (t0 + (int)threadIdx.x < nuniq) tile[threadIdx.x] = s->first[t0 + threadIdx.x];
+    const uint32_t add = t >= d ? sum[t - d] : 0;
     __syncthreads();
-    const int m = min(256, nuniq - t0);
-    for (int q = 0; q < m; ++q) id += tile[q] < r ? 1 : 0;
+    sum[t] += add;
   }
+  uint32_t at = sum[t] - mine;
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    s->start[t * P + q] = s->cursor[t * P + q] = at;
+    at += c[q];
+  }
+  if (t == 1023) s->start[kBuckets] = at;
+}
+
+__global__ void __launch_bounds__(256) k_scatter(Scratch* s, int nuniq, int shift) {
+  const int n = blockIdx.x * 256 + threadIdx.x;
   if (n >= nuniq) return;
-  s->ids[s->slot[n]] = (uint32_t)id;
+  const unsigned long long r = s->first[n];
+  s->sorted[atomicAdd(&s->cursor[r >> shift], 1u)] = r;
+}
+
+// Entry n of the list gets the id that counts the representatives before its own: those of the
+// buckets before its bucket and the smaller ones in it (counting all of them by comparison took
+// 0.17 ms for 32768 materials, as long as the rest of a 32^3 map).
+__global__ void __launch_bounds__(256) k_assign(Coef12 C, Scratch* s, Material* table, int nuniq,
+                                                int shift) {
+  const int n = blockIdx.x * 256 + threadIdx.x;
+  if (n >= nuniq) return;
+  const unsigned long long r = s->first[n];
+  const uint32_t q0 = s->start[r >> shift], q1 = s->start[(r >> shift) + 1];
+  uint32_t id = q0;
+  for (uint32_t q = q0; q < q1; ++q) id += s->sorted[q] < r ? 1u : 0u;
+  s->ids[s->slot[n]] = id;
   float v[12];
 #pragma unroll
   for (int a = 0; a < 12; ++a) v[a] = C.c[a][r];
@@ -250,8 +285,12 @@ cudaError_t build_material_map(const Grid& g, const float* const* coef12, uint16
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   if (hdr[2] != 0 || hdr[0] > (unsigned)kMaxMaterials) return cudaGetLastError();
   const int nuniq = (int)hdr[0];
-  k_list<<<(kSlots + threads - 1) / threads, threads, 0, st>>>(s);
-  k_assign<<<(nuniq + 255) / 256, 256, 0, st>>>(C, s, table, nuniq);
+  int shift = 0;
+  while ((g.plane * g.nz - 1) >> shift >= kBuckets) ++shift;
+  k_list<<<(kSlots + threads - 1) / threads, threads, 0, st>>>(s, shift);
+  k_scan<<<1, 1024, 0, st>>>(s);
+  k_scatter<<<(nuniq + 255) / 256, 256, 0, st>>>(s, nuniq, shift);
+  k_assign<<<(nuniq + 255) / 256, 256, 0, st>>>(C, s, table, nuniq, shift);
   k_map<<<blocks, threads, 0, st>>>(g, C, s, table, mat, n);
   k_mode<<<1, 1024, 0, st>>>(s, (int)hdr[0]);
   unsigned int hdr4[4];

@@ -419,3 +419,31 @@ def test_naive_chunk_lengths_match_oracle(shape, percell):
     assert_fields_match(sim.fields(), oracle.run(shape, coefs, T, sources=[osrc(s) for s in src],
                                                  fields=f), f"naive {shape}")
     sim.close()
+
+
+@pytest.mark.parametrize("shape,where", [((41, 40, 39), "all"), ((97, 95, 71), "first"),
+                                         ((97, 95, 71), "last"), ((64, 61, 33), "none")])
+def test_many_materials_keep_every_tuple(shape, where):
+    """One to 65000 materials, spread over the grid or crowded into its first or last cells (one
+    bucket of the numbering): the coefficients read back and the tiled steps are exact."""
+    nx, ny, nz = shape
+    n, T = nx * ny * nz, 3
+    many = 63000
+    e = np.ones(n, np.float32)
+    distinct = (1.0 + np.random.default_rng(2).permutation(many) / 8192.0).astype(np.float32)
+    at = {"all": np.arange(n) % many, "first": np.minimum(np.arange(n), many - 1),
+          "last": np.maximum(np.arange(n) - (n - many), 0), "none": None}[where]
+    if at is not None:
+        e = distinct[at]
+    coefs = W.reference_coefficients(shape, eps_re=e, t_pml=0)
+    sim = gd.Simulation(*shape, kernel="tiled_w32p", blt=2, tile_rows=32, z_chunks=2)
+    sim.set_coefficients(coefs)
+    assert sim.material_count() == (1 if where == "none" else many)
+    for a, b in zip(sim.get_coefficients(), coefs):
+        assert np.array_equal(a, np.asarray(b).reshape(-1))
+    f = [np.random.default_rng(c).normal(size=n).astype(np.float32) for c in range(6)]
+    for c in range(6):
+        sim.set_field(c, f[c])
+    sim.step(T)
+    assert_fields_match(sim.fields(), oracle.run(shape, coefs, T, fields=f), where)
+    sim.close()
