@@ -19,6 +19,7 @@
 // group of grids of a batch (blockIdx.z = grid).  Monitor values are staged for the deferred DFT.
 // cpml_region recomputes listed cells for the shell companion of the tiled kernel.
 #include <algorithm>
+#include <cstring>
 
 #include "fdtd_kernels.cuh"
 
@@ -447,10 +448,19 @@ __global__ void __launch_bounds__(kHalfThreads, 8) cpml_half(const __grid_consta
   half_block<H>(h, s, t, (int)blockIdx.x, k0, min(h.g.nz, k0 + zc));
 }
 
+// The grids of one launch of a batch.  Every launch, and every node of a captured graph, carries the
+// parameters it is declared with, so there are a few sizes.  Above 4 KB (9 grids) they are dear: a
+// first call of 900 steps captures and starts its graph in 4 to 6 ms for 2 or 8 grids, in 11 ms with
+// the 13 KB of 32 grids (and 14 with the 6.6 KB of 16).
+template <int G>
+struct CpmlGroup {
+  CpmlHot h[G];
+};
+
 // A group of grids of a batch: blockIdx.z = grid of the group.
-template <bool H>
+template <bool H, int G>
 __global__ void __launch_bounds__(kHalfThreads, 8)
-    cpml_half_batch(const __grid_constant__ CpmlGroup grp, const CpmlSim* __restrict__ sims,
+    cpml_half_batch(const __grid_constant__ CpmlGroup<G> grp, const CpmlSim* __restrict__ sims,
                     long long t_offset, int zc) {
   const CpmlHot& h = grp.h[blockIdx.z];
   const CpmlSim& s = sims[blockIdx.z];
@@ -528,25 +538,36 @@ int cpml_planes(long long blocks, int nz) {
   return zc;
 }
 
+template <int G>
+cudaError_t launch_group(const CpmlHot* hot, int n, const CpmlSim* sims, long long t_offset,
+                         int zc, dim3 grd, cudaStream_t st) {
+  CpmlGroup<G> grp;
+  memset(&grp, 0, sizeof(grp));
+  std::copy(hot, hot + n, grp.h);
+  cpml_half_batch<false, G><<<grd, kHalfThreads, 0, st>>>(grp, sims, t_offset, zc);
+  cpml_half_batch<true, G><<<grd, kHalfThreads, 0, st>>>(grp, sims, t_offset, zc);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
-cudaError_t launch_cpml_batch_step(const CpmlGroup& grp, int n, const CpmlSim* sims,
+cudaError_t launch_cpml_batch_step(const CpmlHot* hot, int n, const CpmlSim* sims,
                                    long long t_offset, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (n > kCpmlGroup) return cudaErrorInvalidValue;
   long long blocks = 0;
   int most = 0, max_nz = 0;
   for (int q = 0; q < n; ++q) {
-    const int b = cpml_blocks(grp.h[q]);
+    const int b = cpml_blocks(hot[q]);
     blocks += b;
     most = std::max(most, b);
-    max_nz = std::max(max_nz, grp.h[q].g.nz);
+    max_nz = std::max(max_nz, hot[q].g.nz);
   }
   const int zc = std::max(cpml_planes(blocks, max_nz), (max_nz + 65534) / 65535);
   const dim3 grd((unsigned)most, (unsigned)((max_nz + zc - 1) / zc), (unsigned)n);
-  cpml_half_batch<false><<<grd, kHalfThreads, 0, st>>>(grp, sims, t_offset, zc);
-  cpml_half_batch<true><<<grd, kHalfThreads, 0, st>>>(grp, sims, t_offset, zc);
-  return cudaGetLastError();
+  if (n <= 2) return launch_group<2>(hot, n, sims, t_offset, zc, grd, st);
+  if (n <= 8) return launch_group<8>(hot, n, sims, t_offset, zc, grd, st);
+  return launch_group<kCpmlGroup>(hot, n, sims, t_offset, zc, grd, st);
 }
 
 cudaError_t launch_cpml_step(const CpmlHot& h, const CpmlSim& s, long long t, cudaStream_t st,

@@ -2158,10 +2158,7 @@ fdtd_status batch_step_cpml(fdtd_batch* b, int64_t T, int32_t use_graph, cudaStr
       if (q == T) break;
       for (int g0 = 0; g0 < n; g0 += fdtd::kCpmlGroup) {
         const int ng = std::min(n - g0, fdtd::kCpmlGroup);
-        fdtd::CpmlGroup grp;
-        memset(&grp, 0, sizeof(grp));
-        std::copy(hot.begin() + g0, hot.begin() + g0 + ng, grp.h);
-        BCUDA(b, fdtd::launch_cpml_batch_step(grp, ng, b->d_cpml + g0, q, rs));
+        BCUDA(b, fdtd::launch_cpml_batch_step(hot.data() + g0, ng, b->d_cpml + g0, q, rs));
       }
     }
     return FDTD_OK;

@@ -64,15 +64,12 @@ struct CpmlHot {
 };
 constexpr int kCpmlV = 2;       // consecutive x cells per thread
 constexpr int kCpmlGroup = 32;  // grids per launch of a batch (their CpmlHot are parameters)
-struct CpmlGroup {
-  CpmlHot h[kCpmlGroup];
-};
 // One step of one grid: an E and an H launch.
 cudaError_t launch_cpml_step(const CpmlHot& h, const CpmlSim& s, long long t, cudaStream_t st,
                              int* launches);
-// Step t0 + t_offset of n grids: an E and an H launch (blockIdx.z = grid).  sims: their
-// arguments in device memory.
-cudaError_t launch_cpml_batch_step(const CpmlGroup& grp, int n, const CpmlSim* sims,
+// Step t0 + t_offset of n <= kCpmlGroup grids: an E and an H launch (blockIdx.z = grid).  sims:
+// their arguments in device memory.
+cudaError_t launch_cpml_batch_step(const CpmlHot* hot, int n, const CpmlSim* sims,
                                    long long t_offset, cudaStream_t st);
 // The shell companion of the tiled kernel under CPML layers (cpml.cu): one half step (E, or
 // H with h_half) of step t over the cells of `blocks` (int4 {x tile of 32 cells, y tile of 4

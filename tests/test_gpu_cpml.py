@@ -429,3 +429,22 @@ def test_cpml_chunk_lengths_match_oracle(shape):
                      fields=f)
     assert_fields_match(sim.fields(), F_ref, f"cpml {shape}")
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 17])
+def test_cpml_batches_of_every_parameter_size(n):
+    """Batches up to and past the sizes of a launch's parameter block (2, 8 and 32 grids) equal
+    the grids stepped alone."""
+    rng = np.random.default_rng(n)
+    shapes = [tuple(int(v) for v in rng.integers(12, 25, 3)) for _ in range(n)]
+    sims = [_cpml_sim(s, q % 5, L=4)[0] for q, s in enumerate(shapes)]
+    refs = [_cpml_sim(s, q % 5, L=4)[0] for q, s in enumerate(shapes)]
+    b = gd.Batch(sims)
+    b.step(14)
+    for s, r in zip(sims, refs):
+        r.step(14)
+        s.sync()
+        assert_fields_match(s.fields(), r.fields(), f"{s.shape}")
+    b.close()
+    for s in sims + refs:
+        s.close()
