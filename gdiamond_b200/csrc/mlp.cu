@@ -763,7 +763,7 @@ fdtd_status fdtd_mlp_train(fdtd_mlp* m, int32_t epochs, int32_t batch, float lr,
   // there is room for its workspace; the same results a launch per product at a time otherwise.
   const int steps = (int)((n + mb - 1) / mb);
   const bool fused = m->gemm_kind == FDTD_MLP_GEMM_AUTO &&
-                     fdtd::mlp::train_epoch_supported(m->dims.data(), m->L, mb) &&
+                     fdtd::mlp::train_epoch_supported(m->dims.data(), m->L, mb, (int)m->E) &&
                      epoch_workspace(m, steps);
   fdtd::mlp::TrainArgs ta{};
   std::vector<float2> hc;

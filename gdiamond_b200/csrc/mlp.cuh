@@ -98,8 +98,9 @@ struct TrainArgs {
   const float2* corr;              // [steps]: Adam's bias corrections
   float lr, b1, b2, eps;
 };
-// Hidden and output widths multiples of 16 up to 256, at most 64 inputs and 128 rows a batch.
-bool train_epoch_supported(const int* dims, int L, int batch);
+// Hidden and output widths multiples of 16 up to 256, at most 64 inputs and 128 rows a batch, and no
+// more members than it is the faster path for on the current device.
+bool train_epoch_supported(const int* dims, int L, int batch, int members);
 cudaError_t launch_train_epoch(const TrainArgs& a, int members, cudaStream_t st);
 
 // tcgen05 GEMM (mlp_tc.cu): C[M][N] (+epilogue) for `members` members on `st`; `err` receives

@@ -293,3 +293,19 @@ def test_fused_inference_over_more_rows_than_a_chunk():
             assert rel(a[..., -129:, :], b[..., -129:, :]) <= 1e-3
     for net in nets:
         net.close()
+
+
+@pytest.mark.parametrize("members", [15, 16, 45, 46, 60, 61])
+def test_training_of_large_ensembles_equals_separate_launches(members):
+    """Ensembles whose clusters take turns, on either side of the sizes that go to the separate
+    launches: parameters equal bit for bit."""
+    for dims in ((6, 32, 16), (6, 32, 32, 16)):
+        x, y = data(70, dims, members)
+        got = []
+        for gemm in ("auto", "mma_sync"):
+            net = gd.MLP(dims, members=members, seed=2, gemm=gemm)
+            net.set_data(x, y)
+            net.train(2, batch=32, lr=1e-3, seed=1)
+            got.append(net.get_params())
+            net.close()
+        assert np.array_equal(*got), dims
