@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -441,10 +442,15 @@ std::vector<fdtd::TiledConfig> candidates(const fdtd_handle* h) {
             const int z = (int)((long long)k * nsm / ((long long)gd.x * gd.y));
             if (z > 1 && std::find(zl.begin(), zl.end(), z) == zl.end()) zl.push_back(z);
           }
+          // A chunk shorter than its 2*BLT warm-up is only worth it when asked for; nor are long
+          // chunks while shorter ones still leave no SM with two CTAs.
+          const auto short_chunk = [&](int z) { return (h->g.nz + z - 1) / z < 2 * b; };
+          int full = 0;
+          for (int z : zl)
+            if (!short_chunk(z) && (long long)gd.x * gd.y * z <= nsm) full = std::max(full, z);
           for (int z : zl) {
             c.z_chunks = z;
-            // A chunk shorter than its 2*BLT warm-up is only worth it when asked for.
-            if (!forced_z && (h->g.nz + z - 1) / z < 2 * b) continue;
+            if (!forced_z && (short_chunk(z) || z < full)) continue;
             out.push_back(c);
           }
         }
@@ -492,64 +498,74 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
   cudaEvent_t e0, e1;
   CUDA_TRY(h, cudaEventCreate(&e0));
   CUDA_TRY(h, cudaEventCreate(&e1));
-  // Time one candidate: one untimed launch, then at least `reps` timed launches and `least` ms of
-  // them; ms per step.
-  auto time_cfg = [&](const fdtd::TiledConfig& c, int reps, float least, float* per_step)
-      -> fdtd_status {
+  // Time one candidate: one untimed launch, then `reps` timed ones; ms per step.
+  float launch_ms = 0.1f;  // of the candidate before
+  auto time_cfg = [&](const fdtd::TiledConfig& c, int reps, float* per_step) -> fdtd_status {
     fdtd_status s = ensure_maps(h, c);
     if (s != FDTD_OK) return s;
     fdtd::TiledArgs a = make_tiled_args(h, c, h->t, false);
     a.S = make_sources(h);  // on a small grid the tile with the source ends last
     CUDA_TRY(h, launch_any(c, a, h->g, st));
-    for (int pass = 0; pass < 2; ++pass) {
-      CUDA_TRY(h, cudaEventRecord(e0, st));
-      for (int r = 0; r < reps; ++r) CUDA_TRY(h, launch_any(c, a, h->g, st));
-      CUDA_TRY(h, cudaEventRecord(e1, st));
-      CUDA_TRY(h, cudaEventSynchronize(e1));
-      float ms = 0;
-      CUDA_TRY(h, cudaEventElapsedTime(&ms, e0, e1));
-      *per_step = ms / (reps * c.blt);
-      if (ms >= least) break;
-      reps = std::min(40, (int)(reps * least / std::max(ms, 1e-3f)) + 1);
-    }
+    CUDA_TRY(h, cudaEventRecord(e0, st));
+    for (int r = 0; r < reps; ++r) CUDA_TRY(h, launch_any(c, a, h->g, st));
+    CUDA_TRY(h, cudaEventRecord(e1, st));
+    CUDA_TRY(h, cudaEventSynchronize(e1));
+    float ms = 0;
+    CUDA_TRY(h, cudaEventElapsedTime(&ms, e0, e1));
+    launch_ms = std::max(ms / reps, 1e-3f);
+    *per_step = launch_ms / c.blt;
     return FDTD_OK;
+  };
+  auto launches_for = [](float ms, float one, int least, int most) {
+    return std::min(std::max((int)(ms / one) + 1, least), most);
   };
   // Bring the SM clocks up before anything is compared (an idle GPU starts slow and would
   // penalise whichever candidates run first): launch the first candidate for ~50 ms.
   {
     float warm = 0, spent = 0;
     for (int r = 0; r < 64 && spent < 50.0f; ++r) {
-      fdtd_status s = time_cfg(cands[0], 2, 0.0f, &warm);
+      fdtd_status s = time_cfg(cands[0], 2, &warm);
       if (s != FDTD_OK) return s;
       spent += warm * 2 * cands[0].blt;
     }
   }
-  // First every tile shape at its largest z-chunk count and at 4, then the other counts of the eight
-  // best shapes.
+  // First every tile shape at its largest z-chunk count and at 4 (or its least count above), then the
+  // other counts of the best shapes: ten, within 1.4 times the best, where a launch is short, eight
+  // within 1.35 times where it is not.  (Over 12 grids from 24^3 to 420x400x230 the shape picked in
+  // the end was at most 1.06 from the best there beyond 0.1 ms a launch, 1.30 and in seventh place
+  // below: 100^3.)
   auto shape = [](const fdtd::TiledConfig& c) {
     return std::make_tuple(c.pairs32, c.width, c.rows, c.blt, c.min_blocks);
   };
-  std::map<std::tuple<bool, int, int, int, int>, int> most;  // largest z-chunk count of a shape
-  for (const auto& c : cands) most[shape(c)] = std::max(most[shape(c)], c.z_chunks);
+  std::map<std::tuple<bool, int, int, int, int>, std::pair<int, int>> first;  // the two counts
+  for (const auto& c : cands) {
+    auto& z = first.emplace(shape(c), std::make_pair(INT_MAX, 0)).first->second;
+    if (c.z_chunks >= 4) z.first = std::min(z.first, c.z_chunks);
+    z.second = std::max(z.second, c.z_chunks);
+  }
   std::vector<std::pair<float, size_t>> scored;
   std::vector<bool> timed(cands.size(), false);
   auto score = [&](size_t i) -> fdtd_status {
     float per_step = 0;
     timed[i] = true;
-    fdtd_status s = time_cfg(cands[i], 3, 0.2f, &per_step);
+    fdtd_status s = time_cfg(cands[i], launches_for(0.2f, launch_ms, 3, 8), &per_step);
     if (s == FDTD_OK) scored.emplace_back(per_step, i);
     return s;
   };
-  for (size_t i = 0; i < cands.size(); ++i)
-    if (cands[i].z_chunks == 4 || cands[i].z_chunks == most[shape(cands[i])]) {
-      fdtd_status s = score(i);
-      if (s != FDTD_OK) return s;
-    }
+  for (size_t i = 0; i < cands.size(); ++i) {
+    const auto& z = first[shape(cands[i])];
+    if (cands[i].z_chunks != z.first && cands[i].z_chunks != z.second) continue;
+    fdtd_status s = score(i);
+    if (s != FDTD_OK) return s;
+  }
   std::sort(scored.begin(), scored.end());
   std::vector<std::tuple<bool, int, int, int, int>> top;
+  const bool brief = scored[0].first * cands[scored[0].second].blt <= 0.1f;
   for (const auto& sc : scored) {
     const auto k = shape(cands[sc.second]);
-    if (top.size() < 8 && std::find(top.begin(), top.end(), k) == top.end()) top.push_back(k);
+    if (top.size() < (brief ? 10 : 8) && sc.first <= (brief ? 1.4f : 1.35f) * scored[0].first &&
+        std::find(top.begin(), top.end(), k) == top.end())
+      top.push_back(k);
   }
   for (size_t i = 0; i < cands.size(); ++i)
     if (!timed[i] && std::find(top.begin(), top.end(), shape(cands[i])) != top.end()) {
@@ -564,7 +580,7 @@ fdtd_status autotune(fdtd_handle* h, cudaStream_t st) {
     for (size_t r = 0; r < std::min<size_t>(5, scored.size()); ++r) {
       const fdtd::TiledConfig& c = cands[scored[r].second];
       float per_step = 0;
-      fdtd_status s = time_cfg(c, 8, 0.5f, &per_step);
+      fdtd_status s = time_cfg(c, launches_for(0.5f, scored[r].first * c.blt, 4, 40), &per_step);
       if (s != FDTD_OK) return s;
       if (per_step < best) {
         best = per_step;
