@@ -143,6 +143,7 @@ struct fdtd_handle {
   int maps_key = 0;  // (field box width * 1000 + id box width) * 1000 + rows of the encoded boxes
   int last_kernel = 0, last_launches = 0;
   int last_folds = 0;  // DFT fold launches of the last fdtd_step
+  bool last_own_cfg = false;  // the last fdtd_step ran cpml_companion_config
   int storage = FDTD_STORE_F32;
   int esz = 4;     // bytes per stored field value (F16E: the FP16 E components')
   int nsets = 2;   // field sets (1 for FP64: the naive kernel updates in place)
@@ -179,6 +180,7 @@ struct fdtd_handle {
   long long order_key = -1;
   int version = 0;                 // bumped when coefficients or sources change
   bool lean_ok = false;
+  double lean_share = 0.0;  // share of the blocks that hold the lean material only
   bool lean_enable = true;  // fdtd_set_fast_path
   int lean_id = 0;
   float lean_cb = 0.0f, lean_db = 0.0f;
@@ -728,6 +730,8 @@ fdtd_status compress_coefficients(fdtd_handle* h) {
       CUDA_TRY(h, cudaMemcpyAsync(h->ublk_host.data(), h->ublk, h->ublk_host.size(),
                                   cudaMemcpyDeviceToHost, h->stream));
       CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+      h->lean_share = (double)std::count(h->ublk_host.begin(), h->ublk_host.end(), 1) /
+                      (double)h->ublk_host.size();
     }
   } else {
     h->coef_mode = kCoefPerCell;
@@ -941,12 +945,68 @@ fdtd::CpmlBox cpml_inner_box(const fdtd_handle* h, int r) {
   return b;
 }
 
-// The companion pays off when the inner box of its deepest region still holds most cells.
+// A grid whose caller asks for a temporal block takes the companion when the inner box of its deepest
+// region still holds most cells.
 bool cpml_companion_fits(const fdtd_handle* h, int k) {
   const fdtd::CpmlBox b = cpml_inner_box(h, 3 * k);
   double inner = 1.0;
   for (int a = 0; a < 3; ++a) inner *= (double)(b.hi[a] - b.lo[a]);
   return inner >= 0.4 * (double)h->g.nx * h->g.ny * h->g.nz;
+}
+
+// Whether the tiled kernel with the companion (BLT 2) is expected to be faster than the per-step
+// kernels, by the time a step of either takes on a B200 in us per million cells: the tiled kernel 4.7
+// where all blocks are the lean material, 8.1 where none is (about the square of their share: a tile
+// spans several); the companion 23 of the cells of its blocks, which cover its four regions in two
+// steps; the per-step kernels 12, and 8 more in the layers.  Over 180 grids (64^3 to 850^3, layers of 4
+// to 20 cells on two to six faces, vacuum and mixed) the pick is at most 5 % slower than the other
+// one.  Layers on every face: from 600^3 (4 cells) or 700^3 (10 cells, 4.4 ms a step against 4.7) in
+// vacuum; on the z faces only: from 160^3 (512^3 and 10 cells: 1.0 against 1.6).
+bool cpml_companion_pays(const fdtd_handle* h) {
+  const int n[3] = {h->g.nx, h->g.ny, h->g.nz};
+  const int w[3] = {32, 4, 1};  // cells of a block
+  double blocks = 0, layer = 0;
+  for (int r = 3; r <= 6; ++r) {
+    const fdtd::CpmlBox b = cpml_inner_box(h, r);
+    double all = 1, inside = 1;
+    for (int a = 0; a < 3; ++a) {
+      const int first = (b.lo[a] + w[a] - 1) / w[a];
+      const int last = b.hi[a] == n[a] ? (n[a] + w[a] - 1) / w[a] : b.hi[a] / w[a];
+      all *= (n[a] + w[a] - 1) / w[a];
+      inside *= std::max(0, last - first);
+    }
+    blocks += (all - inside) / 2;
+  }
+  const double cells = 1e-6 * n[0] * n[1] * n[2];
+  for (int a = 0; a < 3; ++a)
+    layer += cells / n[a] * h->cpml.thickness * ((h->cpml_lo[a] ? 1 : 0) + (h->cpml_hi[a] ? 1 : 0));
+  const double lean = h->lean_ok && h->lean_enable ? h->lean_share * h->lean_share : 0.0;
+  const double tiled = 12 + (8.1 - 3.4 * lean) * cells + 23 * 128e-6 * blocks;
+  return tiled < 6 + 12 * cells + 8 * layer;
+}
+
+// The tiled configuration next to the companion when the caller asks for none: 20-row tiles of two
+// CTAs per SM, and the z-chunk count that gives the shortest schedule of full waves (within 2 % of
+// the autotuner's pick from 160^3 to 850^3, without its time: 2.3 s at 700^3).
+fdtd::TiledConfig cpml_companion_config(const fdtd_handle* h) {
+  fdtd::TiledConfig c{2, 20, 1, 32, 1, h->storage, h->esz};
+  c.pairs32 = true;
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->desc.device);
+  long long best = 0;
+  for (int z = 1, pick = 1; z <= std::max(1, h->g.nz / 8) && z <= 64; ++z) {
+    fdtd::TiledConfig t = c;
+    t.z_chunks = z;
+    const dim3 gd = fdtd::tiled2_grid(t, h->g);
+    const long long waves = ((long long)gd.x * gd.y * gd.z + 2 * nsm - 1) / (2 * nsm);
+    const long long time = waves * ((h->g.nz + z - 1) / z + 2 * c.blt);
+    if (best == 0 || time < best) {
+      best = time;
+      pick = z;
+    }
+    c.z_chunks = pick;
+  }
+  return c;
 }
 
 // Device list of the 32 x 4-cell blocks (x tile, y tile, plane) that hold cells of W_r.
@@ -980,20 +1040,41 @@ fdtd_status cpml_region_blocks(fdtd_handle* h, int r, std::pair<int4*, int>* out
   return FDTD_OK;
 }
 
+// The companion's third field set (all six or none).
+fdtd_status cpml_companion_fields(fdtd_handle* h) {
+  if (h->cpml_scratch[0]) return FDTD_OK;
+  for (int c = 0; c < 6; ++c)
+    if (cudaMalloc(&h->cpml_scratch[c], h->cells * sizeof(float)) != cudaSuccess) {
+      for (int q = 0; q < 6; ++q) {
+        cudaFree(h->cpml_scratch[q]);
+        h->cpml_scratch[q] = nullptr;
+      }
+      cudaGetLastError();
+      return fail(h, FDTD_ERR_OOM, "CPML companion field set allocation failed");
+    }
+  return FDTD_OK;
+}
+
+// Whether there is room for the companion of launches of up to two steps.
+bool cpml_companion_room(fdtd_handle* h) {
+  if (cpml_companion_fields(h) != FDTD_OK) return false;
+  std::pair<int4*, int> list;
+  for (int r = 2; r <= 6; ++r)  // 3 k - 2 (j - 1) and one less: 3, 2 and 6, 5, 4, 3
+    if (cpml_region_blocks(h, r, &list) != FDTD_OK) {
+      cudaGetLastError();
+      cpml_release_companion(h);
+      return false;
+    }
+  return true;
+}
+
 // The companion of one tiled launch of k steps from field set `src` (step t) to `dst`.
 fdtd_status cpml_companion(fdtd_handle* h, int k, int src, int dst, long long t,
                            const fdtd::Sources& S, const fdtd::Monitors& M, cudaStream_t st,
                            int* launches) {
-  if (k > 1 && !h->cpml_scratch[0]) {  // all six or none
-    for (int c = 0; c < 6; ++c)
-      if (cudaMalloc(&h->cpml_scratch[c], h->cells * sizeof(float)) != cudaSuccess) {
-        for (int q = 0; q < 6; ++q) {
-          cudaFree(h->cpml_scratch[q]);
-          h->cpml_scratch[q] = nullptr;
-        }
-        cudaGetLastError();
-        return fail(h, FDTD_ERR_OOM, "CPML companion field set allocation failed");
-      }
+  if (k > 1) {
+    const fdtd_status s = cpml_companion_fields(h);
+    if (s != FDTD_OK) return s;
   }
   fdtd::FieldPtrs A, B, C;
   for (int c = 0; c < 6; ++c) {
@@ -1392,11 +1473,11 @@ fdtd_status fdtd_step(fdtd_handle* h, int64_t T, void* stream) {
   }
   fdtd_status s = ensure_tables(h, h->t + T);
   if (s != FDTD_OK) return s;
-  // CPML layers: one E and one H kernel per step over the whole grid, monitors staged; or, when
-  // the caller asks for a temporal block (desc.blt) and the grid is large enough for it, the tiled
-  // kernel with the shell companion.  The companion recomputes a third of a 256^3 grid with
-  // 10-cell layers and was the slower of the two there (0.45 against 0.30 ms a step).
-  bool companion = false;
+  // CPML layers: one E and one H kernel per step over the whole grid, monitors staged; or the tiled
+  // kernel with the shell companion, when the caller asks for a temporal block (desc.blt) and the
+  // grid is large enough for it, or asks for no tile shape at all and the companion is expected to
+  // be faster and has room.
+  bool companion = false, own_cfg = false;
   if (h->cpml_on) {
     if (h->storage != FDTD_STORE_F32)
       return fail(h, FDTD_ERR_UNSUPPORTED, "CPML layers need FP32 field storage");
@@ -1404,6 +1485,10 @@ fdtd_status fdtd_step(fdtd_handle* h, int64_t T, void* stream) {
         h->coef_mode == kCoefMaterial && cpml_companion_fits(h, 1)) {
       if (!h->cfg_ready && (s = autotune(h, st)) != FDTD_OK) return s;
       companion = cpml_companion_fits(h, h->cfg.blt);
+    } else if ((h->desc.kernel == FDTD_KERNEL_AUTO || h->desc.kernel == FDTD_KERNEL_TILED) &&
+               h->desc.blt == 0 && h->desc.tile_rows == 0 && h->desc.z_chunks == 0 &&
+               h->desc.min_blocks == 0 && h->coef_mode == kCoefMaterial && cpml_companion_pays(h)) {
+      companion = own_cfg = cpml_companion_room(h);
     }
   }
   if (h->cpml_on && !companion) {
@@ -1424,6 +1509,7 @@ fdtd_status fdtd_step(fdtd_handle* h, int64_t T, void* stream) {
     }
     if (sim.M.n > 0 && h->t > t_fold && (s = fold()) != FDTD_OK) return s;
     h->last_kernel = 6;  // reported by fdtd_get_config: the per-step CPML kernels
+    h->last_own_cfg = false;
     h->last_launches = launches;
     h->last_folds = folds;
     if (st != h->stream) {
@@ -1460,11 +1546,11 @@ fdtd_status fdtd_step(fdtd_handle* h, int64_t T, void* stream) {
     }
     h->last_kernel = FDTD_KERNEL_NAIVE;
   } else {
-    if (!h->cfg_ready) {
+    if (!own_cfg && !h->cfg_ready) {
       s = autotune(h, st);
       if (s != FDTD_OK) return s;
     }
-    fdtd::TiledConfig c = h->cfg;
+    fdtd::TiledConfig c = own_cfg ? cpml_companion_config(h) : h->cfg;
     c.storage = h->storage;  // the kernel instance must match this handle's field storage
     c.esz = h->esz;
     s = ensure_maps(h, c);
@@ -1506,6 +1592,7 @@ fdtd_status fdtd_step(fdtd_handle* h, int64_t T, void* stream) {
     h->last_kernel = c.pairs32 ? FDTD_KERNEL_TILED_W32P
                                : (c.width == 64 ? FDTD_KERNEL_TILED_W64 : FDTD_KERNEL_TILED_W32);
   }
+  h->last_own_cfg = own_cfg;
   h->last_launches = launches;
   h->last_folds = folds;
   if (st != h->stream) {
@@ -1883,12 +1970,13 @@ fdtd_status fdtd_dft_folds(const fdtd_handle* h, int32_t* n) {
 
 fdtd_status fdtd_get_config(const fdtd_handle* h, int32_t* out6) {
   if (!h || !out6) return FDTD_ERR_INVALID_ARG;
+  const fdtd::TiledConfig c = h->last_own_cfg ? cpml_companion_config(h) : h->cfg;
   out6[0] = h->last_kernel;
-  out6[1] = h->cfg.blt;
-  out6[2] = h->cfg.rows;
-  out6[3] = h->cfg.z_chunks;
+  out6[1] = c.blt;
+  out6[2] = c.rows;
+  out6[3] = c.z_chunks;
   out6[4] = h->last_launches;
-  out6[5] = h->cfg.min_blocks;
+  out6[5] = c.min_blocks;
   return FDTD_OK;
 }
 
@@ -2220,6 +2308,7 @@ fdtd_status batch_step_cpml(fdtd_batch* b, int64_t T, int32_t use_graph, cudaStr
   for (fdtd_handle* h : b->sims) {
     h->t += T;
     h->last_kernel = 6;  // the per-step CPML kernels
+    h->last_own_cfg = false;
     h->last_launches = launches;
     h->last_folds = folds;
     fdtd_status r = stream_after(b, h->stream, st);
@@ -2401,6 +2490,7 @@ fdtd_status fdtd_batch_step(fdtd_batch* b, int64_t T, int32_t use_graph, void* s
     h->t += T;
     h->cur ^= (nl & 1);
     h->last_kernel = c.pairs32 ? FDTD_KERNEL_TILED_W32P : FDTD_KERNEL_TILED_W64;
+    h->last_own_cfg = false;
     h->last_launches = nl;
     h->last_folds = folds;
     if ((s = stream_after(b, h->stream, st)) != FDTD_OK) return s;

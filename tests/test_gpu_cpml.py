@@ -448,3 +448,85 @@ def test_cpml_batches_of_every_parameter_size(n):
     b.close()
     for s in sims + refs:
         s.close()
+
+
+def _long_column(kernel, t_pml=0):
+    """A grid whose z layers are a small part of it: the default route is the tiled kernel with
+    the shell companion."""
+    shape = (96, 90, 641)
+    sim = gd.Simulation(*shape, kernel=kernel)
+    sim.set_permittivity(None, t_pml=t_pml)
+    sim.set_cpml(thickness=7, faces=16 | 32, kappa_max=1.5)
+    w = W.gaussian_wave(60, delay=6.0, width=3.0, period=5.0)
+    sim.set_sources([dict(component="Jx", wave=w, k=9, kind=gd.SRC_PLANE_Z),
+                     dict(component="Jz", wave=w, i=40, j=33, k=3),
+                     dict(component="Jy", wave=w, i=41, j=30, k=320)])
+    f = np.random.default_rng(0).normal(size=shape[0] * shape[1] * shape[2]).astype(np.float32)
+    for c in range(6):
+        sim.set_field(c, np.roll(f, 1000 * c))
+    mid = sim.add_dft_monitor("Ez", 5, W.source_band(4, period=5.0, width=3.0))
+    return sim, mid
+
+
+def test_cpml_default_route_of_thin_layers_matches_per_step_path():
+    """Bit for bit over an odd number of steps (a last launch of one), before and after a reset and
+    with the fast path off (a different estimate of the tiled kernel)."""
+    (sim, sm), (ref, rm) = _long_column("auto"), _long_column("naive")
+    for n, T in enumerate((5, 24)):
+        for s in (sim, ref):
+            s.step(T)
+            s.sync()
+        assert ref.config()["kernel"] == "cpml"
+        assert sim.config()["kernel"] == "tiled" and sim.config()["blt"] == 2
+        assert_fields_match(sim.fields(), ref.fields(), f"default route, call {n}")
+        for a, b in zip(sim.get_dft(sm) + tuple(sim.cpml_state()),
+                        ref.get_dft(rm) + tuple(ref.cpml_state())):
+            assert np.array_equal(a, b)
+    for s in (sim, ref):
+        s.reset()
+        s.set_fast_path(False)
+        s.step(7)
+    assert_fields_match(sim.fields(), ref.fields(), "default route after a reset")
+    sim.close()
+    ref.close()
+
+
+def test_cpml_default_route_without_room_steps_all_the_same():
+    """The companion needs a third field set; without room for it the per-step kernels, which do
+    not, take the steps."""
+    import ctypes
+    (sim, _), (ref, _) = _long_column("auto"), _long_column("naive")
+    for s in (sim, ref):
+        s.sync()
+    ref.step(9)  # its kernels are loaded; the monitors' tables come first in both
+    ref.sync()
+    sim.step(1)
+    sim.sync()
+    assert sim.config()["kernel"] == "tiled"
+    sim.set_cpml(thickness=7, faces=16 | 32, kappa_max=1.5)  # gives the third set back
+    sim.reset()
+    ref.reset()
+    rt = ctypes.CDLL([q.split()[-1] for q in open("/proc/self/maps") if "libcudart.so" in q][0])
+    hold = []
+    for size in (1 << 30, 1 << 26, 1 << 21):
+        p = ctypes.c_void_p()
+        while rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0:
+            hold.append(p)
+            p = ctypes.c_void_p()
+        rt.cudaGetLastError()
+    try:
+        sim.step(9)
+        sim.sync()
+        assert sim.config()["kernel"] == "cpml"
+        ref.step(9)
+        ref.sync()
+    finally:
+        for p in hold:
+            rt.cudaFree(p)
+    sim.step(3)
+    ref.step(3)
+    sim.sync()
+    assert sim.config()["kernel"] == "tiled"  # there is room again
+    assert_fields_match(sim.fields(), ref.fields(), "without room")
+    sim.close()
+    ref.close()
