@@ -13,9 +13,8 @@
 //
 // A thread owns two plane cells and kFoldF frequencies: their sums stay in registers for the whole
 // window, the staged values of consecutive cells are coalesced, and each (cos, sin) pair of a
-// step, a broadcast load, serves both cells.  Bound: FP64 issue.
-#include <type_traits>
-
+// step, a broadcast load, serves both cells.  Bound: FP64 issue with many monitors or frequencies,
+// the latency of a step's loads with few (256 x 256 cells, 8 frequencies: 256 blocks, 7 warps per SM).
 #include "fdtd_kernels.cuh"
 
 namespace fdtd {
@@ -27,21 +26,22 @@ constexpr int kFoldF = 8;  // frequencies per thread
 
 constexpr int kFoldP = 2;  // plane cells per thread, kFoldThreads apart
 
-__device__ __forceinline__ void fold_monitor(const MonitorDev& m, const Grid& g, long long t0,
-                                             int n) {
-  const long long np = (long long)g.nx * g.ny;
-  const long long p0 = (long long)blockIdx.x * (kFoldThreads * kFoldP) + threadIdx.x;
-  const int f0 = (int)blockIdx.y * kFoldF;
-  if (m.stage == nullptr || p0 >= np || f0 >= m.nf) return;
+// Adds n staged steps from t0 on to the sums of NF frequencies from f0 on, for the plane cells p[].
+// NF is a constant: a run-time count splits the step into a branch per frequency, with no independent
+// work between them (5 frequencies of 6 monitors of 400 x 400 cells: 1.46 ms a window of 128 steps with
+// a run-time count, 0.87 with constants).
+template <int NF, bool SCALED>
+__device__ __forceinline__ void fold_cells(const MonitorDev& m, long long np,
+                                           const long long (&p)[kFoldP], bool two, int f0,
+                                           long long t0, int n) {
+  // (always NF; as a run-time guard of the first loads it makes the compiler keep the loop's registers
+  // apart from theirs: without it 8 frequencies take 1.3 times as long)
   const int nfc = min(kFoldF, m.nf - f0);
-  // a thread without a second cell folds its first one twice and stores it once
-  const bool two = p0 + kFoldThreads < np;
-  const long long p[kFoldP] = {p0, two ? p0 + kFoldThreads : p0};
-  double re[kFoldP][kFoldF], im[kFoldP][kFoldF];
+  double re[kFoldP][NF], im[kFoldP][NF];
 #pragma unroll
   for (int c = 0; c < kFoldP; ++c)
 #pragma unroll
-    for (int q = 0; q < kFoldF; ++q) {
+    for (int q = 0; q < NF; ++q) {
       re[c][q] = q < nfc ? m.re[(long long)(f0 + q) * np + p[c]] : 0.0;
       im[c][q] = q < nfc ? m.im[(long long)(f0 + q) * np + p[c]] : 0.0;
     }
@@ -51,46 +51,67 @@ __device__ __forceinline__ void fold_monitor(const MonitorDev& m, const Grid& g,
   const int nf = m.nf;
   const double2* tab0 = m.tab + t0 * nf + f0;
   const int slot0 = (int)(t0 & (kDftSlots - 1));
-  // x * 1.0 == x: without a scale two of the six operations per step and frequency fall away.
-  auto window = [&](auto scaled, auto full) {
 #pragma unroll 2
-    for (int s = 0; s < n; ++s) {
-      const long long o = (long long)((slot0 + s) & (kDftSlots - 1)) * np;
-      const double v[kFoldP] = {(double)st0[o], (double)st1[o]};
-      const double2* tab = tab0 + (long long)s * nf;
+  for (int s = 0; s < n; ++s) {
+    const long long o = (long long)((slot0 + s) & (kDftSlots - 1)) * np;
+    const double v[kFoldP] = {(double)st0[o], (double)st1[o]};
+    const double2* tab = tab0 + (long long)s * nf;
 #pragma unroll
-      for (int q = 0; q < kFoldF; ++q) {
-        if (decltype(full)::value || q < nfc) {
-          const double2 cs = __ldg(&tab[q]);
+    for (int q = 0; q < NF; ++q) {
+      const double2 cs = __ldg(&tab[q]);
 #pragma unroll
-          for (int k = 0; k < kFoldP; ++k) {
-            double c = dmul(v[k], cs.x), d = dmul(v[k], cs.y);
-            if (decltype(scaled)::value) {
-              c = dmul(c, scale);
-              d = dmul(d, scale);
-            }
-            re[k][q] = dadd(re[k][q], c);
-            im[k][q] = dsub(im[k][q], d);
-          }
+      for (int k = 0; k < kFoldP; ++k) {
+        double c = dmul(v[k], cs.x), d = dmul(v[k], cs.y);
+        if (SCALED) {
+          c = dmul(c, scale);
+          d = dmul(d, scale);
         }
+        re[k][q] = dadd(re[k][q], c);
+        im[k][q] = dsub(im[k][q], d);
       }
     }
-  };
-  using Yes = std::true_type;
-  using No = std::false_type;
-  if (scale == 1.0) {
-    if (nfc == kFoldF) window(No{}, Yes{}); else window(No{}, No{});
-  } else {
-    if (nfc == kFoldF) window(Yes{}, Yes{}); else window(Yes{}, No{});
   }
 #pragma unroll
   for (int c = 0; c < kFoldP; ++c)
 #pragma unroll
-    for (int q = 0; q < kFoldF; ++q)
-      if (q < nfc && (c == 0 || two)) {
+    for (int q = 0; q < NF; ++q)
+      if (c == 0 || two) {
         m.re[(long long)(f0 + q) * np + p[c]] = re[c][q];
         m.im[(long long)(f0 + q) * np + p[c]] = im[c][q];
       }
+}
+
+template <int NF>
+__device__ __forceinline__ void fold_group(const MonitorDev& m, long long np,
+                                           const long long (&p)[kFoldP], bool two, int f0,
+                                           long long t0, int n) {
+  // x * 1.0 == x: without a scale two of the six operations per step and frequency fall away
+  if (m.scale == 1.0)
+    fold_cells<NF, false>(m, np, p, two, f0, t0, n);
+  else
+    fold_cells<NF, true>(m, np, p, two, f0, t0, n);
+}
+
+__device__ __forceinline__ void fold_monitor(const MonitorDev& m, const Grid& g, long long t0,
+                                             int n) {
+  const long long np = (long long)g.nx * g.ny;
+  const long long p0 = (long long)blockIdx.x * (kFoldThreads * kFoldP) + threadIdx.x;
+  const int f0 = (int)blockIdx.y * kFoldF;
+  if (m.stage == nullptr || p0 >= np || f0 >= m.nf) return;
+  // a thread without a second cell folds its first one twice and stores it once
+  const bool two = p0 + kFoldThreads < np;
+  const long long p[kFoldP] = {p0, two ? p0 + kFoldThreads : p0};
+  static_assert(kFoldF == 8, "the cases below");
+  switch (min(kFoldF, m.nf - f0)) {
+    case 1: fold_group<1>(m, np, p, two, f0, t0, n); break;
+    case 2: fold_group<2>(m, np, p, two, f0, t0, n); break;
+    case 3: fold_group<3>(m, np, p, two, f0, t0, n); break;
+    case 4: fold_group<4>(m, np, p, two, f0, t0, n); break;
+    case 5: fold_group<5>(m, np, p, two, f0, t0, n); break;
+    case 6: fold_group<6>(m, np, p, two, f0, t0, n); break;
+    case 7: fold_group<7>(m, np, p, two, f0, t0, n); break;
+    default: fold_group<8>(m, np, p, two, f0, t0, n); break;
+  }
 }
 
 // One grid: blockIdx.z is the monitor.
@@ -99,8 +120,9 @@ __global__ void __launch_bounds__(kFoldThreads) dft_fold(const __grid_constant__
   if ((int)blockIdx.z < M.n) fold_monitor(M.m[blockIdx.z], g, t0, n);
 }
 
-// A batch: blockIdx.z is grid * kMaxMonitors + monitor; the grid's arguments (monitors, step counter t0 at the start of the
-// batch step) are the ones the batched kernel reads (TiledArgs, or CpmlSim for CPML batches).
+// A batch: blockIdx.z is grid * kMaxMonitors + monitor; the grid's arguments (monitors, step counter
+// t0 at the start of the batch step) are the ones the batched kernel reads (TiledArgs, or CpmlSim for
+// CPML batches).
 // The window starts t_offset steps later.
 template <class Args>
 __global__ void __launch_bounds__(kFoldThreads) dft_fold_batch(const Args* grids,

@@ -447,3 +447,22 @@ def test_many_materials_keep_every_tuple(shape, where):
     sim.step(T)
     assert_fields_match(sim.fields(), oracle.run(shape, coefs, T, fields=f), where)
     sim.close()
+
+
+@pytest.mark.parametrize("shape", [(11, 11, 7), (19, 7, 9), (37, 9, 9)])
+def test_dft_folds_of_every_frequency_count(shape):
+    """1 to 17 frequencies (every size of a thread's last group), with and without a scale, planes
+    of one cell to two cells a thread: sums bit for bit over a window and a short one."""
+    T = 131
+    coefs = W.vacuum_coefficients(shape)
+    w = W.gaussian_wave(T, delay=9.0, width=4.0, period=7.0)
+    sources = [dict(component="Jz", wave=w, i=shape[0] // 2, j=shape[1] // 2, k=shape[2] // 2)]
+    for nfs in ((1, 2, 3, 4, 5, 6, 7, 8, 9), (10, 11, 12, 13, 14, 15, 16, 17)):
+        mons = [dict(component=("Ez", "Hy")[n % 2], k=shape[2] // 2, scale=(1.0, 0.3)[n % 3 == 0],
+                     freqs=W.source_band(n, period=7.0, width=4.0)) for n in nfs]
+        omons = [oracle.Monitor(m["component"], m["k"], m["freqs"], m["scale"]) for m in mons]
+        oracle.run(shape, coefs, T, sources=[osrc(s) for s in sources], monitors=omons)
+        _, D, _ = gpu_run(shape, coefs, T, sources, mons, kernel="tiled_w32p", blt=2, tile_rows=20,
+                          z_chunks=1, min_blocks=1)
+        for m, o, (re, im) in zip(mons, omons, D):
+            assert np.array_equal(re, o.re) and np.array_equal(im, o.im), len(m["freqs"])
