@@ -113,6 +113,17 @@ struct Store<__nv_bfloat16> {
   }
 };
 
+// CTAs per SM the compiler must fit at least: two for the 20- and 24-row tiles of 32-cell rows (320
+// and 384 threads), and for 256 threads (8 rows of 64 cells) where the compiler left to itself takes
+// more than the 128 registers of two CTAs: at BLT 3 (137 of them: 96 us a step of 160x150x140 vacuum,
+// 67 with 128) and in batches (126 to 178); one otherwise.
+constexpr int tiled2_min_blocks(int rows, int w, int blt, bool batch) {
+  return (w == 32 && (rows == 20 || rows == 24)) ||
+                 (rows * w / 2 <= 256 && (blt == 3 || batch))
+             ? 2
+             : 1;
+}
+
 // W = 64: one 64-cell row per warp (32 lanes x an x-pair).  W = 32: two 32-cell rows per warp
 // (16 lanes x an x-pair each), so a CTA of the same 16 warps covers a 32 x 32 tile instead of
 // 64 x 16: more of it valid under the trapezoid and a finer x granularity on small grids.
@@ -668,7 +679,9 @@ __device__ __forceinline__ Smem setup_smem(unsigned char* smem_raw, int* s_abort
 // One grid: one tile per CTA.  MINB > 1 caps registers so that MINB CTAs fit on an SM (more
 // warps to hide latency, at the cost of some spilled state); the autotuner decides.
 template <typename S, int B, int TY, int MINB, int W = 64, typename SH = S>
-__global__ void __launch_bounds__(TY * W / 2, MINB)
+__global__ void __launch_bounds__(TY * W / 2, (tiled2_min_blocks(TY, W, B, false) > MINB
+                                                     ? tiled2_min_blocks(TY, W, B, false)
+                                                     : MINB))
     fdtd_tiled2(const __grid_constant__ TiledArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_abort;
@@ -687,16 +700,9 @@ __global__ void __launch_bounds__(TY * W / 2, MINB)
     (void)march<S, B, TY, W, SH, false>(a, bx, by, bz, sm, gbase, 0);
 }
 
-// CTAs per SM the compiler must fit: two for the 20- and 24-row tiles of 32-cell rows (320 and
-// 384 threads), one otherwise.
-template <int TY, int W>
-constexpr int batch_min_blocks() {
-  return (W == 32 && (TY == 20 || TY == 24)) ? 2 : 1;
-}
-
 // A batch of independent grids: persistent CTAs pull (grid, tile) work items from a queue.
 template <typename S, int B, int TY, int W = 64, typename SH = S>
-__global__ void __launch_bounds__(TY * W / 2, (batch_min_blocks<TY, W>()))
+__global__ void __launch_bounds__(TY * W / 2, tiled2_min_blocks(TY, W, B, true))
     fdtd_tiled2_batch(const BatchArgs b) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_abort;
