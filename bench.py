@@ -347,7 +347,7 @@ def run_ours(args):
     sim.set_coefficients(coefs)
     sim.set_fast_path(not args.no_fast_path)
     if args.cpml:
-        # per-step kernels, or with --blt the tiled kernel plus the shell companion
+        # per-step kernels; the tiled kernel plus the shell companion with --blt or thin layers
         sim.set_cpml(thickness=args.cpml)
     sim.set_sources(src)
     mid = sim.add_dft_monitor("Ez", nz // 2, freqs, scale=1.0)
@@ -1138,7 +1138,8 @@ def main():
                          "an independent replica per GPU")
     ap.add_argument("--cpml", type=int, default=0,
                     help="CPML layers of this many cells on every face (the per-step E/H "
-                         "kernels instead of the tiled kernel)")
+                         "kernels instead of the tiled kernel, except for thin layers around "
+                         "large grids)")
     ap.add_argument("--no-fast-path", action="store_true",
                     help="force the general per-cell path of the x-pair kernels")
     ap.add_argument("--workload", default="plain",

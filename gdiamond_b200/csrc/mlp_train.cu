@@ -6,7 +6,7 @@
 // microsecond of work.  Here a cluster of 16 CTAs (8 for more than 4 members) takes one member
 // through every minibatch of the epoch.  The members are independent, so nothing waits outside
 // its cluster.  4 members of 6-256-256-256-64, 4096 rows in batches of 64: 37 us a step instead of
-// 154 (8 CTAs 58, 16 CTAs of 256 threads 45); bound by the latency of the chain (issue slots 27 %
+// 154 (8 CTAs 58, 16 CTAs of 256 threads 45); bound by the latency of the chain (issue slots 38 %
 // busy, fixed-latency and barrier stalls).
 //
 // Split: CTA c owns a slice of 16-column groups of every layer's outputs.  It computes those
